@@ -34,6 +34,7 @@
 #include <climits>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -791,12 +792,26 @@ __global__ void k_wait_selftest(const int4 *__restrict__ src, unsigned long long
 // A level whose sliced copy fits in the shared memory of a cluster of at most
 // kClusterMax CTAs runs all its sweeps (and the residual after them) in one
 // launch: CTA q loads slices [q spc, (q + 1) spc) -- values, explicit
-// columns, metadata, f, d and its rows of the iterate -- once, and every pass
-// reads the iterate of the other CTAs through distributed shared memory, with
-// a cluster barrier between passes.  The row sums repeat slice_row_sum
-// operation for operation (same gather indices, same partial sums, same
-// batch size), so the results are those of the separate launches bit for
-// bit, while the level costs one launch instead of one per pass.
+// columns, metadata, f and d -- once, with a cluster barrier between passes.
+// The iterate lives in shared memory in one of two ways:
+//   distributed (copies made of offset slices): a CTA holds its own rows and
+//     gathers the others' through distributed shared memory; a stencil's
+//     gathers are contiguous 32-row segments, few of them remote;
+//   replicated (copies with column slices): every CTA holds the whole
+//     iterate, gathers from its own memory, and stores each new row into
+//     every CTA's other copy (a contiguous 32-row store per CTA).
+// What bounds a pass is the traffic between the SMs (about 14 bytes per
+// clock and SM).  On unordered rows almost every gather of the distributed
+// form is a remote access per lane, 32 bytes of traffic each: one pass over
+// the coarsest level of a random geometric graph (2,601 rows, 17.6 slots
+// wide, FP32) took 12.5 us distributed and takes 1.9 us replicated, and 2,145
+// rows in FP64 12.7 us and 2.2 us.  Replication moves every row to every CTA
+// instead, so for stencils, whose gathers are mostly local, it is the slower
+// form (7-point, 8,192 rows, FP64: 1.75 us distributed, 2.4 us replicated).
+// The row sums repeat the row pass operation for operation (same gather
+// indices, same partial sums, same batch size), so the results are those of
+// separate launches bit for bit, while the level costs one launch instead of
+// one per pass.
 namespace cg = cooperative_groups;
 
 constexpr int kClusterWarps = 16;
@@ -809,17 +824,20 @@ constexpr size_t kClusterSmem = 220 * 1024;
 constexpr int32_t kClusterWarpSlots = 32;
 
 // One CTA's shared memory: the same offsets in every CTA of the cluster, so
-// a remote CTA's iterate sits where the local one does.
+// a remote CTA's iterate sits where the local one does.  xslices: slices of
+// the iterate that a CTA holds (its own, or all of them when replicated).
 struct ClusterLayout {
   uint32_t vals, cols, meta, x0, x1, f, d, bytes;
-  __host__ __device__ ClusterLayout(int slots, int vbytes, bool cols_on, int spc, int xbytes) {
+  __host__ __device__ ClusterLayout(int slots, int vbytes, bool cols_on, int spc, int xslices,
+                                    int xbytes) {
     vals = 0;
     cols = vals + ((static_cast<uint32_t>(slots) * 32u * vbytes + 15u) & ~15u);
     meta = cols + (cols_on ? static_cast<uint32_t>(slots) * 32u * 4u : 0u);
     const uint32_t rows = static_cast<uint32_t>(spc) * 32u * xbytes;
+    const uint32_t xrows = static_cast<uint32_t>(xslices) * 32u * xbytes;
     x0 = meta + static_cast<uint32_t>(spc) * 16u;
-    x1 = x0 + rows;
-    f = x1 + rows;
+    x1 = x0 + xrows;
+    f = x1 + xrows;
     d = f + rows;
     bytes = d + rows;
   }
@@ -834,10 +852,10 @@ struct ClusterArgs {
   int zero_start;
 };
 
-// Gathers from the iterate held across the cluster's shared memory: row j
-// lives in CTA j >> shift at position j & mask.
+// Gathers from the iterate distributed over the cluster's shared memory: row
+// j lives in CTA j >> shift at position j & mask.
 template <typename XT>
-struct ClusterGather {
+struct DistributedGather {
   XT *xc;
   int shift;
   int32_t mask, r;
@@ -851,33 +869,60 @@ struct ClusterGather {
   __device__ XT rel_param(int32_t o) const { return (*this)(r + o); }
 };
 
-template <typename VT, typename XT, int KB>
+// Gathers from the CTA's own copy of the whole iterate.
+template <typename XT>
+struct ReplicatedGather {
+  const XT *x;
+  const XT *xr;
+  __device__ void row(int32_t r) { xr = x + r; }
+  __device__ XT operator()(int32_t i) const { return x[i]; }
+  __device__ XT rel(int32_t o) const { return xr[o]; }
+  __device__ XT rel_param(int32_t o) const { return xr[o]; }
+};
+
+// Shared-memory address of the same variable in CTA `rank` of the cluster,
+// and a store to it.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+
+template <typename VT, typename XT, int KB, bool Repl>
 __global__ void __launch_bounds__(kClusterThreads)
     k_sl_cluster(SlicedView S, ClusterArgs<XT> a) {
-  pdl_wait();
-  pdl_trigger();
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(128) unsigned char smem[];
-  const ClusterLayout L(S.cl_slots, sizeof(VT), S.cols_staged != 0, S.cl_spc, sizeof(XT));
+  const ClusterLayout L(S.cl_slots, sizeof(VT), S.cols_staged != 0, S.cl_spc,
+                        Repl ? S.nslices : S.cl_spc, sizeof(XT));
   __shared__ __align__(8) uint64_t loaded;
-  const int q = static_cast<int>(cl.block_rank());
+  const int q = static_cast<int>(cl.block_rank()), nq = static_cast<int>(cl.num_blocks());
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  // slices per CTA are a power of two: a row's owner is a shift away
+  // distributed: slices per CTA are a power of two, a row's owner a shift away
   const int32_t spc = S.cl_spc, rows_cta = spc * 32;
   const int rshift = __ffs(rows_cta) - 1;
   const int32_t s0 = min(q * spc, S.nslices), s1 = min(s0 + spc, S.nslices);
   const int32_t r0 = s0 * 32, nrow = max(0, min(s1 * 32, S.n) - r0);
-  const int32_t p0 = S.sptr[s0], p1 = S.sptr[s1];
+  const int32_t x_first = Repl ? 0 : r0;  // row at the start of this CTA's iterate
   VT *sv = reinterpret_cast<VT *>(smem + L.vals);
   int32_t *sc = reinterpret_cast<int32_t *>(smem + L.cols);
   int4 *sm = reinterpret_cast<int4 *>(smem + L.meta);
   XT *xb0 = reinterpret_cast<XT *>(smem + L.x0), *xb1 = reinterpret_cast<XT *>(smem + L.x1);
   XT *sf = reinterpret_cast<XT *>(smem + L.f), *sd = reinterpret_cast<XT *>(smem + L.d);
   const VT *val = static_cast<const VT *>(S.val);
+  const int32_t p0 = S.sptr[s0], p1 = S.sptr[s1];
   // The CTA's slots plus the padding a batch may read past its last slice
   // (the global copy is padded the same way; those values are never used),
   // its columns and metadata: bulk async copies under one mbarrier (all
-  // 16-byte multiples at 16-byte aligned addresses).
+  // 16-byte multiples at 16-byte aligned addresses).  The matrix copy was
+  // complete before the kernel ahead of this one started, so these loads
+  // need not wait for that kernel (pdl_wait below) and overlap its end.
   const uint32_t nsl = static_cast<uint32_t>(p1 - p0 + kSlotPad) * 32u;
   if (tid == 0) {
     mbar_init(&loaded, 1);
@@ -889,13 +934,28 @@ __global__ void __launch_bounds__(kClusterThreads)
     if (cbytes) bulk_load(sc, S.scol + static_cast<int64_t>(p0) * 32, cbytes, &loaded);
     bulk_load(sm, S.meta + s0, mbytes, &loaded);
   }
+  pdl_wait();
+  pdl_trigger();
+  // Before a remote store: every CTA of the cluster has started.  (The
+  // barrier also orders the mbarrier's initialisation before the waits.)
+  if (Repl) cl.sync();
   for (int32_t i = tid; i < nrow; i += kClusterThreads) {
     const XT fi = a.f[r0 + i], di = a.d[r0 + i];
     sf[i] = fi;
     sd[i] = di;
-    xb0[i] = a.zero_start ? fi / di : a.u[r0 + i];
+    if (!Repl) {
+      xb0[i] = a.zero_start ? fi / di : a.u[r0 + i];
+    } else if (a.zero_start) {
+      const uint32_t at = smem_addr(xb0 + r0 + i);
+      const XT v = fi / di;
+      for (int t = 0; t < nq; ++t) cluster_store(cluster_addr(at, t), v);
+    }
   }
-  __syncthreads();  // (the barrier's initialisation before anyone waits on it)
+  if (Repl && !a.zero_start) {
+#pragma unroll 8
+    for (int32_t i = tid; i < S.n; i += kClusterThreads) xb0[i] = a.u[i];
+  }
+  __syncthreads();
   if (!mbar_wait(&loaded, 0, kDrainLimitNs)) atomicExch(&g_sliced_wait_error, 1);
   cl.sync();
   const int32_t hi = S.n - 1;
@@ -906,7 +966,11 @@ __global__ void __launch_bounds__(kClusterThreads)
     const bool resid = p == sweeps;
     XT *xc = cur ? xb1 : xb0;
     XT *xn = cur ? xb0 : xb1;
-    ClusterGather<XT> gath{xc, rshift, rows_cta - 1, 0};
+    std::conditional_t<Repl, ReplicatedGather<XT>, DistributedGather<XT>> gath;
+    if constexpr (Repl)
+      gath = {xc, xc};
+    else
+      gath = {xc, rshift, rows_cta - 1, 0};
     for (int32_t ls = wid; ls < s1 - s0; ls += kClusterWarps) {
       const int4 m = sm[ls];
       const int32_t r = (s0 + ls) * 32 + lane;
@@ -916,18 +980,25 @@ __global__ void __launch_bounds__(kClusterThreads)
                             : row_sum<VT, XT, KB>(sv + rel, m.z ? nullptr : sc + rel,
                                                   S.soff + m.w, m.y, r, hi, m.z == 2, gath);
       if (r < S.n) {
-        const int32_t rl = r - r0;
-        if (resid)
+        const int32_t rl = r - r0, xi = r - x_first;
+        if (resid) {
           a.res[r] = sf[rl] - T;
-        else
-          xn[rl] = ((-T + sf[rl]) / sd[rl]) + xc[rl];
+        } else {
+          const XT v = ((-T + sf[rl]) / sd[rl]) + xc[xi];
+          if (Repl) {
+            const uint32_t at = smem_addr(xn + xi);
+            for (int t = 0; t < nq; ++t) cluster_store(cluster_addr(at, t), v);
+          } else {
+            xn[xi] = v;
+          }
+        }
       }
     }
     cl.sync();  // every read of this pass's iterate is done before the next
     if (!resid) cur ^= 1;
   }
   const XT *xf = cur ? xb1 : xb0;
-  for (int32_t i = tid; i < nrow; i += kClusterThreads) a.u[r0 + i] = xf[i];
+  for (int32_t i = tid; i < nrow; i += kClusterThreads) a.u[r0 + i] = xf[r0 - x_first + i];
 }
 
 // ---- launch configuration ----------------------------------------------------
@@ -1026,10 +1097,10 @@ bcmg_status pipe_launch(const SlicedView &S, const XT *x, const Epi &epi, cudaSt
 // gather batch chosen as pipe_launch chooses it (the partial sums depend on
 // it).  The shared-memory attribute is set on first use, which sliced_build
 // makes happen outside any stream capture.
-template <typename VT, typename XT, int KB>
-bcmg_status cluster_launch_kb(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
+template <typename VT, typename XT, int KB, bool Repl>
+bcmg_status cluster_launch_as(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
                               bool warm_only) {
-  auto kern = k_sl_cluster<VT, XT, KB>;
+  auto kern = k_sl_cluster<VT, XT, KB, Repl>;
   {
     static std::mutex mu;
     static bool attr_set = false;
@@ -1041,7 +1112,8 @@ bcmg_status cluster_launch_kb(const SlicedView &S, const ClusterArgs<XT> &a, cud
     }
   }
   if (warm_only) return BCMG_OK;
-  const ClusterLayout L(S.cl_slots, sizeof(VT), S.cols_staged != 0, S.cl_spc, sizeof(XT));
+  const ClusterLayout L(S.cl_slots, sizeof(VT), S.cols_staged != 0, S.cl_spc,
+                        Repl ? S.nslices : S.cl_spc, sizeof(XT));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S.cl_size);
   cfg.blockDim = dim3(kClusterThreads);
@@ -1059,6 +1131,14 @@ bcmg_status cluster_launch_kb(const SlicedView &S, const ClusterArgs<XT> &a, cud
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
   BCMG_CUDA(cudaLaunchKernelEx(&cfg, kern, S, a));
   return BCMG_OK;
+}
+
+// Copies with column slices keep the iterate replicated (see above).
+template <typename VT, typename XT, int KB>
+bcmg_status cluster_launch_kb(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
+                              bool warm_only) {
+  return S.cols_staged ? cluster_launch_as<VT, XT, KB, true>(S, a, st, warm_only)
+                       : cluster_launch_as<VT, XT, KB, false>(S, a, st, warm_only);
 }
 
 template <typename VT, typename XT>
@@ -1181,8 +1261,12 @@ bcmg_status plan_cluster(SlicedMat *out, cudaStream_t s) {
     BCMG_CUDA(cudaMemcpyAsync(h_sptr.data(), out->sptr, sizeof(int32_t) * (ns + 1),
                               cudaMemcpyDeviceToHost, s));
     BCMG_CUDA(cudaStreamSynchronize(s));
-    int32_t spc = 1;  // a power of two with at most kClusterMax CTAs
-    while (static_cast<int64_t>(spc) * kClusterMax < ns) spc <<= 1;
+    const bool repl = out->has_columns;
+    int32_t spc = ceil_div(ns, kClusterMax);
+    if (!repl) {  // a power of two: the owner of a row is a shift away
+      spc = 1;
+      while (static_cast<int64_t>(spc) * kClusterMax < ns) spc <<= 1;
+    }
     const int32_t csize = ceil_div(ns, spc);
     int32_t cap = 0, warp_slots = 0;
     for (int32_t q = 0; q < csize; ++q) {
@@ -1195,8 +1279,8 @@ bcmg_status plan_cluster(SlicedMat *out, cudaStream_t s) {
       }
     }
     cap += kSlotPad;
-    const ClusterLayout CL(cap, static_cast<int>(value_bytes(out->vtype)), out->has_columns, spc,
-                           out->xtype == kValF64 ? 8 : 4);
+    const ClusterLayout CL(cap, static_cast<int>(value_bytes(out->vtype)), repl, spc,
+                           repl ? ns : spc, out->xtype == kValF64 ? 8 : 4);
     if (CL.bytes <= kClusterSmem && warp_slots <= kClusterWarpSlots) {
       out->cl_size = csize;
       out->cl_spc = spc;
