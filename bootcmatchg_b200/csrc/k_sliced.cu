@@ -472,7 +472,7 @@ __device__ __forceinline__ XT stencil_row_sum(const VT *v, const SlicedView &S, 
 template <typename XT>
 struct EpiRelax {  // out = ((-T + f) / d) + u
   static constexpr int NV = 3;
-  __device__ bool active() const { return true; }
+  static constexpr bool kGated = false;
   const XT *f, *d, *u;
   XT *out;
   __device__ const XT *row_vec(int i) const { return i == 0 ? f : (i == 1 ? d : u); }
@@ -484,7 +484,7 @@ struct EpiRelax {  // out = ((-T + f) / d) + u
 // sweep of the mixed cycle, which hands its result to FP64 vectors).
 struct EpiRelaxWiden {  // out = double(((-T + f) / d) + u)
   static constexpr int NV = 3;
-  __device__ bool active() const { return true; }
+  static constexpr bool kGated = false;
   const float *f, *d, *u;
   double *out;
   __device__ const float *row_vec(int i) const { return i == 0 ? f : (i == 1 ? d : u); }
@@ -497,7 +497,7 @@ struct EpiRelaxWiden {  // out = double(((-T + f) / d) + u)
 template <typename XT>
 struct EpiResidual {  // out = f - T
   static constexpr int NV = 1;
-  __device__ bool active() const { return true; }
+  static constexpr bool kGated = false;
   const XT *f;
   XT *out;
   __device__ const XT *row_vec(int) const { return f; }
@@ -508,7 +508,7 @@ struct EpiResidual {  // out = f - T
 template <typename XT>
 struct EpiSpmvT {  // out = T
   static constexpr int NV = 0;
-  __device__ bool active() const { return true; }
+  static constexpr bool kGated = false;
   XT *out;
   __device__ const XT *row_vec(int) const { return nullptr; }
   __device__ void apply(int32_t r, XT T, const XT *) { out[r] = T; }
@@ -520,7 +520,7 @@ using EpiSpmv = EpiSpmvT<double>;
 // vector); per-CTA partial sums in warp order, written to partials[4 b + k].
 struct EpiFcgDots {
   static constexpr int NV = 3;
-  __device__ bool active() const { return true; }
+  static constexpr bool kGated = false;
   const double *v, *r, *q;  // q == nullptr: no gamma
   double *w, *partials;
   double acc[3];
@@ -561,6 +561,7 @@ struct EpiReplace {
   double *r, *partials;
   const double *scal;
   double acc[1];
+  static constexpr bool kGated = true;  // runs only if active()
   __device__ bool active() const { return scal[kReplace] != 0.0; }
   __device__ const double *row_vec(int) const { return b; }
   __device__ void apply(int32_t row, double T, const double *rv) {
@@ -614,19 +615,25 @@ constexpr int pipe_min_blocks() {
   return sizeof(XT) == 8 ? 3 : (KB >= 27 ? kWideMinBlocks : 4);
 }
 
+// What the kernel reads of the matrix copy (slot bounds, values, columns,
+// metadata) was complete before the kernel ahead of it started, so the
+// producer fills its first stages with it before pdl_wait(); only the row
+// vectors and the gathers wait for that kernel.
 template <typename VT, typename XT, typename Epi, int KB>
 __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
     k_sl_pipe(SlicedView S, const VT *__restrict__ val, const XT *__restrict__ x, Epi epi,
               int cap_slots, int cols_staged) {
-  pdl_wait();
-  pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kPipeStages], empty[kPipeStages];
   __shared__ StageCtl ctl[kPipeStages];
   constexpr int NVS = Epi::NV > 0 ? Epi::NV : 1;
-  if (!epi.active()) return;  // uniform: a device flag read by every thread
+  if constexpr (Epi::kGated) {
+    pdl_wait();
+    if (!epi.active()) return;  // uniform: a device flag read by every thread
+  }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int32_t nchunks = (S.nslices + kPipeWarps - 1) / kPipeWarps;
+  const int32_t c_first = blockIdx.x, c_last = nchunks, c_step = gridDim.x;
   const StageLayout L(cap_slots, sizeof(VT), sizeof(XT), cols_staged != 0, Epi::NV);
   if (threadIdx.x == 0) {
     for (int i = 0; i < kPipeStages; ++i) {
@@ -644,48 +651,68 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
     bool rows_aligned = Epi::NV > 0;
     for (int i = 0; i < Epi::NV; ++i)
       rows_aligned = rows_aligned && (reinterpret_cast<uintptr_t>(epi.row_vec(i)) & 15u) == 0;
-    int32_t c = blockIdx.x;
-    int32_t p0 = c < nchunks ? __ldg(S.sptr + c * kPipeWarps) : 0;
-    int32_t p1 = c < nchunks ? __ldg(S.sptr + min((c + 1) * kPipeWarps, S.nslices)) : 0;
-    int j = 0;
-    for (; c < nchunks; ++j, c += gridDim.x) {
-      const int32_t cn = c + gridDim.x;  // next chunk's bounds, loaded ahead
-      const int32_t q0 = cn < nchunks ? __ldg(S.sptr + cn * kPipeWarps) : 0;
-      const int32_t q1 = cn < nchunks ? __ldg(S.sptr + min((cn + 1) * kPipeWarps, S.nslices)) : 0;
-      const int st = j % kPipeStages;
-      if (j >= kPipeStages &&
-          !mbar_wait(&empty[st], static_cast<uint32_t>(((j / kPipeStages) - 1) & 1),
-                     S.wait_ns)) {
-        atomicExch(&g_sliced_wait_error, 1);
-        break;
-      }
+    // The rows of chunk c and whether their vectors are staged.
+    auto chunk_rows = [&](int32_t c, int32_t *r0) -> uint32_t {
+      const int32_t s1 = min((c + 1) * kPipeWarps, S.nslices);
+      *r0 = c * kPipeWarps * 32;
+      const uint32_t rbytes = static_cast<uint32_t>(min(s1 * 32, S.n) - *r0) * sizeof(XT);
+      return rows_aligned && (rbytes % 16u) == 0 ? rbytes : 0u;
+    };
+    auto load_rows = [&](int32_t c, int st) {
+      int32_t r0;
+      const uint32_t rbytes = chunk_rows(c, &r0);
+      if (!rbytes || !((armed >> st) & 1u)) return;
+      unsigned char *rows = smem + static_cast<size_t>(st) * L.bytes + L.rows;
+      for (int i = 0; i < Epi::NV; ++i)
+        bulk_load(rows + i * kPipeWarps * 32 * sizeof(XT), epi.row_vec(i) + r0, rbytes,
+                  &full[st]);
+    };
+    // Arms the stage for chunk c (slots [p0, p1)) and copies its part of the
+    // matrix; load_rows completes it.
+    auto load_matrix = [&](int32_t c, int st, int32_t p0, int32_t p1) {
       const int32_t s0 = c * kPipeWarps, s1 = min(s0 + kPipeWarps, S.nslices);
-      const int32_t r0 = s0 * 32, r1 = min(s1 * 32, S.n);
-      const uint32_t rbytes = static_cast<uint32_t>(r1 - r0) * sizeof(XT);
-      const bool rows_ok = rows_aligned && (rbytes % 16u) == 0;
+      int32_t r0;
+      const uint32_t rbytes = chunk_rows(c, &r0);
       const bool fits = p1 - p0 <= cap_slots;
       ctl[st].slot0 = p0;
       ctl[st].staged = fits;
-      ctl[st].rows_staged = rows_ok;
+      ctl[st].rows_staged = rbytes != 0;
       unsigned char *base = smem + static_cast<size_t>(st) * L.bytes;
       if (fits) {
         const uint32_t nsl = static_cast<uint32_t>(p1 - p0) * 32u;
         const uint32_t vb = nsl * sizeof(VT);
         const uint32_t cb = cols_staged ? nsl * 4u : 0u;
         const uint32_t mb = static_cast<uint32_t>(s1 - s0) * 16u;
-        mbar_arrive_tx(&full[st], vb + cb + mb + (rows_ok ? Epi::NV * rbytes : 0u));
+        mbar_arrive_tx(&full[st], vb + cb + mb + Epi::NV * rbytes);
         if (vb) bulk_load(base + L.vals, val + static_cast<int64_t>(p0) * 32, vb, &full[st]);
         if (cb) bulk_load(base + L.cols, S.scol + static_cast<int64_t>(p0) * 32, cb, &full[st]);
         bulk_load(base + L.meta, S.meta + s0, mb, &full[st]);
-        if (rows_ok)
-          for (int i = 0; i < Epi::NV; ++i)
-            bulk_load(base + L.rows + i * kPipeWarps * 32 * sizeof(XT), epi.row_vec(i) + r0,
-                      rbytes, &full[st]);
         armed |= 1u << st;
       } else {
         armed &= ~(1u << st);
         mbar_arrive(&full[st]);
       }
+    };
+    auto slot_at = [&](int32_t c) { return __ldg(S.sptr + min(c * kPipeWarps, S.nslices)); };
+    int j = 0;
+    int32_t c = c_first;
+    for (; j < kPipeStages && c < c_last; ++j, c += c_step)
+      load_matrix(c, j, slot_at(c), slot_at(c + 1));
+    if constexpr (!Epi::kGated) pdl_wait();
+    for (int i = 0; i < j; ++i) load_rows(c_first + i * c_step, i);
+    int32_t p0 = c < c_last ? slot_at(c) : 0, p1 = c < c_last ? slot_at(c + 1) : 0;
+    for (; c < c_last; ++j, c += c_step) {
+      const int32_t cn = c + c_step;  // next chunk's bounds, loaded ahead
+      const int32_t q0 = cn < c_last ? slot_at(cn) : 0;
+      const int32_t q1 = cn < c_last ? slot_at(cn + 1) : 0;
+      const int st = j % kPipeStages;
+      if (!mbar_wait(&empty[st], static_cast<uint32_t>(((j / kPipeStages) - 1) & 1),
+                     S.wait_ns)) {
+        atomicExch(&g_sliced_wait_error, 1);
+        break;
+      }
+      load_matrix(c, st, p0, p1);
+      load_rows(c, st);
       p0 = q0;
       p1 = q1;
     }
@@ -703,9 +730,11 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
   }
 
   // consumers
+  if constexpr (!Epi::kGated) pdl_wait();
+  pdl_trigger();
   const int32_t hi = S.n - 1;
-  int32_t c = blockIdx.x;
-  for (int j = 0; c < nchunks; ++j, c += gridDim.x) {
+  int32_t c = c_first;
+  for (int j = 0; c < c_last; ++j, c += c_step) {
     const int st = j % kPipeStages;
     if (!mbar_wait_warp(&full[st], static_cast<uint32_t>((j / kPipeStages) & 1),
                         S.wait_ns)) {
