@@ -127,8 +127,7 @@ __global__ void k_slice_shape(int32_t n, int32_t nslices, const int32_t *__restr
 }
 
 // Format statistics from the scanned slot pointers: stats[0] = the most slots
-// in one chunk of kPipeWarps slices, stats[1] = 1 if any slice is a column
-// slice.
+// in one chunk of kPipeWarps slices, stats[1] = the slots of column slices.
 __global__ void k_slice_stats(int32_t nslices, const int32_t *__restrict__ sptr,
                               const int32_t *__restrict__ kind, int32_t *stats) {
   const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -136,11 +135,10 @@ __global__ void k_slice_stats(int32_t nslices, const int32_t *__restrict__ sptr,
   if (s0 >= nslices) return;
   const int32_t s1 = min(s0 + kPipeWarps, nslices);
   atomicMax(stats, sptr[s1] - sptr[s0]);
+  int32_t col_slots = 0;
   for (int32_t s = s0; s < s1; ++s)
-    if (!kind[s]) {
-      atomicOr(stats + 1, 1);
-      break;
-    }
+    if (!kind[s]) col_slots += sptr[s + 1] - sptr[s];
+  if (col_slots) atomicAdd(stats + 1, col_slots);
 }
 
 // Which narrower types hold every value exactly (bitwise round trip):
@@ -472,7 +470,7 @@ __device__ __forceinline__ XT stencil_row_sum(const VT *v, const SlicedView &S, 
 template <typename XT>
 struct EpiRelax {  // out = ((-T + f) / d) + u
   static constexpr int NV = 3;
-  static constexpr bool kGated = false;
+  static constexpr bool kGated = false, kPartials = false;
   const XT *f, *d, *u;
   XT *out;
   __device__ const XT *row_vec(int i) const { return i == 0 ? f : (i == 1 ? d : u); }
@@ -484,7 +482,7 @@ struct EpiRelax {  // out = ((-T + f) / d) + u
 // sweep of the mixed cycle, which hands its result to FP64 vectors).
 struct EpiRelaxWiden {  // out = double(((-T + f) / d) + u)
   static constexpr int NV = 3;
-  static constexpr bool kGated = false;
+  static constexpr bool kGated = false, kPartials = false;
   const float *f, *d, *u;
   double *out;
   __device__ const float *row_vec(int i) const { return i == 0 ? f : (i == 1 ? d : u); }
@@ -497,7 +495,7 @@ struct EpiRelaxWiden {  // out = double(((-T + f) / d) + u)
 template <typename XT>
 struct EpiResidual {  // out = f - T
   static constexpr int NV = 1;
-  static constexpr bool kGated = false;
+  static constexpr bool kGated = false, kPartials = false;
   const XT *f;
   XT *out;
   __device__ const XT *row_vec(int) const { return f; }
@@ -508,7 +506,7 @@ struct EpiResidual {  // out = f - T
 template <typename XT>
 struct EpiSpmvT {  // out = T
   static constexpr int NV = 0;
-  static constexpr bool kGated = false;
+  static constexpr bool kGated = false, kPartials = false;
   XT *out;
   __device__ const XT *row_vec(int) const { return nullptr; }
   __device__ void apply(int32_t r, XT T, const XT *) { out[r] = T; }
@@ -520,7 +518,7 @@ using EpiSpmv = EpiSpmvT<double>;
 // vector); per-CTA partial sums in warp order, written to partials[4 b + k].
 struct EpiFcgDots {
   static constexpr int NV = 3;
-  static constexpr bool kGated = false;
+  static constexpr bool kGated = false, kPartials = true;
   const double *v, *r, *q;  // q == nullptr: no gamma
   double *w, *partials;
   double acc[3];
@@ -562,6 +560,7 @@ struct EpiReplace {
   const double *scal;
   double acc[1];
   static constexpr bool kGated = true;  // runs only if active()
+  static constexpr bool kPartials = true;
   __device__ bool active() const { return scal[kReplace] != 0.0; }
   __device__ const double *row_vec(int) const { return b; }
   __device__ void apply(int32_t row, double T, const double *rv) {
@@ -787,6 +786,113 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
   epi.finish(wid, lane);
 }
 
+// ---- row passes of column-slice copies ------------------------------------
+// Rows with unordered columns: a gather of the iterate touches up to 32
+// sectors, so a pass is bound by the gathers an SM keeps in flight and by
+// L1's rate for them (about one sector per clock: 45 us for the 12.8 M
+// entries of a 1 M-node random geometric graph), not by the value stream.
+// The staged pipeline above holds only 8 to 16 consumer warps per SM on such
+// copies (two stages of 55 to 63 KB at 8 bytes per entry).  This kernel
+// stages nothing: one warp per slice, 24 (FP32 vectors) or 16 (FP64) warps
+// per SM, kColBatch gathers in flight per lane.  The slices of a warp run as
+// one sequence of batches, so the next batch's columns -- of the same slice
+// or of the warp's next one -- load while the current gathers are in flight.
+// Fewer gathers (8) with more warps were slower: the register budget then
+// spilled.  Values and columns are read once per pass (__ldcs).  Per sweep,
+// staged and here: 1 M nodes, FP32, 20.6 slots, 81.4 and 54.1 us; its second
+// level (272 K rows) 43.8 and 18.3; 300 K nodes, FP64, 28.1 and 20.7; 2-D
+// finite volume, third level, 108 K rows, BF16, 10 slots, 3.7 and 2.8.
+// Slots are summed in four partial sums by slot index mod 4, as row_sum does
+// for any batch that is a multiple of four (slot_batch).  Loads ahead stay
+// inside the padded column array, and every stored column is in range
+// (padding slots hold the row itself or zero).
+constexpr int kColBatch = 12;  // gathers in flight per lane
+
+template <typename VT, typename XT, typename Epi>
+__global__ void __launch_bounds__(kPipeWarps * 32, sizeof(XT) == 8 ? 2 : 3)
+    k_sl_cols(SlicedView S, const VT *__restrict__ val, const XT *__restrict__ x, Epi epi) {
+  constexpr int NVS = Epi::NV > 0 ? Epi::NV : 1, KB = kColBatch;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int32_t hi = S.n - 1, step = gridDim.x * kPipeWarps;
+  int32_t s = blockIdx.x * kPipeWarps + wid;
+  // The matrix copy was complete before the kernel ahead of this one started
+  // (see k_sl_pipe): its first loads need not wait for that kernel.
+  int4 m = __ldg(S.meta + min(s, S.nslices - 1));
+  int32_t cc[KB];
+  {
+    const int32_t *c = S.scol + static_cast<int64_t>(m.x) * 32 + lane;
+#pragma unroll
+    for (int q = 0; q < KB; ++q) cc[q] = __ldcs(c + q * 32);
+  }
+  pdl_wait();
+  pdl_trigger();
+  if constexpr (Epi::kGated)
+    if (!epi.active()) return;
+  while (s < S.nslices) {
+    const int32_t r = s * 32 + lane;
+    XT rv[NVS];
+#pragma unroll
+    for (int i = 0; i < NVS; ++i) rv[i] = XT(0);
+    if (r < S.n) {
+#pragma unroll
+      for (int i = 0; i < Epi::NV; ++i) rv[i] = epi.row_vec(i)[r];
+    }
+    const int4 mn = __ldg(S.meta + min(s + step, S.nslices - 1));
+    const int64_t at = static_cast<int64_t>(m.x) * 32 + lane;
+    const int32_t *cnext = S.scol + static_cast<int64_t>(mn.x) * 32 + lane;
+    XT T;
+    if (m.z == 0) {
+      XT t[4] = {XT(0), XT(0), XT(0), XT(0)};
+      const int W = m.y;
+      const VT *v = val + at;
+      const int32_t *c = S.scol + at;
+      int k = 0;
+      do {
+        VT vv[KB];
+        XT xv[KB];
+        const bool last = k + KB >= W;
+        const int32_t *cp = last ? cnext : c + (k + KB) * 32;
+        if (k + KB <= W) {
+#pragma unroll
+          for (int q = 0; q < KB; ++q) xv[q] = __ldg(x + cc[q]);
+#pragma unroll
+          for (int q = 0; q < KB; ++q) vv[q] = __ldcs(v + (k + q) * 32);
+#pragma unroll
+          for (int q = 0; q < KB; ++q) cc[q] = __ldcs(cp + q * 32);
+#pragma unroll
+          for (int q = 0; q < KB; ++q)
+            t[q & 3] = fma(static_cast<XT>(widen(vv[q])), xv[q], t[q & 3]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < KB; ++q)
+            if (k + q < W) xv[q] = __ldg(x + cc[q]);
+#pragma unroll
+          for (int q = 0; q < KB; ++q)
+            if (k + q < W) vv[q] = __ldcs(v + (k + q) * 32);
+#pragma unroll
+          for (int q = 0; q < KB; ++q) cc[q] = __ldcs(cp + q * 32);
+#pragma unroll
+          for (int q = 0; q < KB; ++q)
+            if (k + q < W) t[q & 3] = fma(static_cast<XT>(widen(vv[q])), xv[q], t[q & 3]);
+        }
+        k += KB;
+      } while (k < W);
+      T = (t[0] + t[1]) + (t[2] + t[3]);
+    } else {
+      GlobalGather<XT> g{x, x};
+      g.row(r);
+      T = row_sum<VT, XT, KB>(val + at, nullptr, S.soff + __ldg(S.meta + s).w, m.y, r, hi,
+                              m.z >= 2, g);
+#pragma unroll
+      for (int q = 0; q < KB; ++q) cc[q] = __ldcs(cnext + q * 32);
+    }
+    if (r < S.n) epi.apply(r, T, rv);
+    s += step;
+    m = mn;
+  }
+  epi.finish(wid, lane);
+}
+
 // Self-test of the bounded pipeline waits with the pipeline's own wait
 // functions: one CTA; lane 0 of warp 0 (the producer) stages one real bulk
 // copy on barrier 0 and drains it; warp 1 (a consumer) waits on barrier 1,
@@ -850,7 +956,12 @@ constexpr size_t kClusterSmem = 220 * 1024;
 // A pass costs about one dependent shared-memory gather chain per slot of
 // the busiest warp; beyond this many slots a separate launch per sweep over
 // the whole GPU is faster (27-point stencils: one 32-row slice per warp).
-constexpr int32_t kClusterWarpSlots = 32;
+// Gathers of the CTA's own memory are cheaper, so the replicated form takes
+// twice as many.
+constexpr int32_t kClusterWarpSlots = 32, kClusterWarpSlotsRepl = 64;
+// The replicated form also stops where its stores to the other CTAs cost as
+// much as a launch: an iterate of this many bytes.
+constexpr int64_t kClusterReplBytes = 24 * 1024;
 
 // One CTA's shared memory: the same offsets in every CTA of the cluster, so
 // a remote CTA's iterate sits where the local one does.  xslices: slices of
@@ -1042,7 +1153,8 @@ struct PipeCfg {
 // once per kernel and size, outside any stream capture: sliced_build warms
 // the cache for the kernels a matrix will use).
 template <typename K>
-bcmg_status pipe_cfg(K kernel, size_t stage_bytes, int32_t nchunks, PipeCfg *out) {
+bcmg_status pipe_cfg(K kernel, int threads, size_t stage_bytes, int32_t nchunks, PipeCfg *out,
+                     bool partials) {
   static std::mutex mu;
   static std::map<std::pair<const void *, size_t>, int> cache;
   const size_t smem = kPipeStages * stage_bytes;
@@ -1056,10 +1168,11 @@ bcmg_status pipe_cfg(K kernel, size_t stage_bytes, int32_t nchunks, PipeCfg *out
     } else {
       // Always the largest size any matrix may ask for, so a later matrix
       // never lowers the limit another one relies on.
-      BCMG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(kPipeStages * kMaxStageBytes)));
-      BCMG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPipeThreads,
-                                                              smem));
+      if (smem)
+        BCMG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(kPipeStages * kMaxStageBytes)));
+      BCMG_CUDA(
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
       if (per_sm < 1) return set_error(BCMG_ERR_INTERNAL, "sliced pipeline does not fit an SM");
       cache[key] = per_sm;
     }
@@ -1067,9 +1180,9 @@ bcmg_status pipe_cfg(K kernel, size_t stage_bytes, int32_t nchunks, PipeCfg *out
   int dev = 0, sms = kNumSM;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // At most kRedBlocks CTAs: the FCG epilogue writes one partial per CTA.
-  out->grid = static_cast<int>(std::min<int64_t>(
-      std::min<int64_t>(nchunks, static_cast<int64_t>(per_sm) * sms), kRedBlocks));
+  out->grid = static_cast<int>(std::min<int64_t>(nchunks, static_cast<int64_t>(per_sm) * sms));
+  // At most kRedBlocks CTAs where the epilogue writes one partial sum per CTA.
+  if (partials) out->grid = std::min(out->grid, kRedBlocks);
   out->smem = smem;
   return BCMG_OK;
 }
@@ -1080,7 +1193,10 @@ bcmg_status pipe_cfg(K kernel, size_t stage_bytes, int32_t nchunks, PipeCfg *out
 // gathers per batch (two batches cover a 27-point row), which keeps three
 // CTAs per SM in the register file.  The summation order depends on KB, so
 // every kernel reading a copy uses this rule.
-inline int slot_batch(int32_t batch, bool f64) {
+// Copies whose slots are mostly column slots run k_sl_cols; there any multiple
+// of four gives its order, and 8 suits the cluster's gathers from shared memory.
+inline int slot_batch(int32_t batch, bool f64, bool direct) {
+  if (direct) return 8;
   if (batch <= 5) return 5;
   if (batch <= 7) return 7;
   if (batch <= 8) return 8;
@@ -1098,17 +1214,27 @@ bcmg_status pipe_launch(const SlicedView &S, const XT *x, const Epi &epi, cudaSt
                         bool warm_only = false) {
   if (S.nslices <= 0) return BCMG_OK;
   const int32_t nchunks = ceil_div(S.nslices, kPipeWarps);
-  const StageLayout L(S.cap_slots, sizeof(VT), sizeof(XT), S.cols_staged != 0, Epi::NV);
   PipeCfg cfg;
+  if (S.direct) {
+    auto kern = k_sl_cols<VT, XT, Epi>;
+    BCMG_TRY(pipe_cfg(kern, kPipeWarps * 32, 0, nchunks, &cfg, Epi::kPartials));
+    if (!warm_only) {
+      launch_pdl(kern, cfg.grid, kPipeWarps * 32, 0, st, S, static_cast<const VT *>(S.val), x,
+                 epi);
+      BCMG_LAUNCH_CHECK();
+    }
+    return BCMG_OK;
+  }
+  const StageLayout L(S.cap_slots, sizeof(VT), sizeof(XT), S.cols_staged != 0, Epi::NV);
 #define BCMG_PIPE_KB(KB_)                                                                   \
   do {                                                                                      \
     auto kern = k_sl_pipe<VT, XT, Epi, KB_>;                                                \
-    BCMG_TRY(pipe_cfg(kern, L.bytes, nchunks, &cfg));                                       \
+    BCMG_TRY(pipe_cfg(kern, kPipeThreads, L.bytes, nchunks, &cfg, Epi::kPartials));                                       \
     if (!warm_only)                                                                         \
       launch_pdl(kern, cfg.grid, kPipeThreads, cfg.smem, st, S, static_cast<const VT *>(S.val), \
              x, epi, S.cap_slots, S.cols_staged);                                           \
   } while (0)
-  switch (slot_batch(S.batch, sizeof(XT) == 8)) {
+  switch (slot_batch(S.batch, sizeof(XT) == 8, S.direct != 0)) {
     case 5: BCMG_PIPE_KB(5); break;
     case 7: BCMG_PIPE_KB(7); break;
     case 8: BCMG_PIPE_KB(8); break;
@@ -1173,7 +1299,7 @@ bcmg_status cluster_launch_kb(const SlicedView &S, const ClusterArgs<XT> &a, cud
 template <typename VT, typename XT>
 bcmg_status cluster_launch(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
                            bool warm_only = false) {
-  switch (slot_batch(S.batch, sizeof(XT) == 8)) {
+  switch (slot_batch(S.batch, sizeof(XT) == 8, S.direct != 0)) {
     case 5: return cluster_launch_kb<VT, XT, 5>(S, a, st, warm_only);
     case 7: return cluster_launch_kb<VT, XT, 7>(S, a, st, warm_only);
     case 8: return cluster_launch_kb<VT, XT, 8>(S, a, st, warm_only);
@@ -1182,7 +1308,7 @@ bcmg_status cluster_launch(const SlicedView &S, const ClusterArgs<XT> &a, cudaSt
   if constexpr (sizeof(XT) == 8) {
     return cluster_launch_kb<VT, XT, 14>(S, a, st, warm_only);
   } else {
-    switch (slot_batch(S.batch, false)) {
+    switch (slot_batch(S.batch, false, S.direct != 0)) {
       case 16: return cluster_launch_kb<VT, XT, 16>(S, a, st, warm_only);
       case 27: return cluster_launch_kb<VT, XT, 27>(S, a, st, warm_only);
       default: return cluster_launch_kb<VT, XT, 28>(S, a, st, warm_only);
@@ -1310,7 +1436,11 @@ bcmg_status plan_cluster(SlicedMat *out, cudaStream_t s) {
     cap += kSlotPad;
     const ClusterLayout CL(cap, static_cast<int>(value_bytes(out->vtype)), repl, spc,
                            repl ? ns : spc, out->xtype == kValF64 ? 8 : 4);
-    if (CL.bytes <= kClusterSmem && warp_slots <= kClusterWarpSlots) {
+    const bool pays = repl ? warp_slots <= kClusterWarpSlotsRepl &&
+                                 static_cast<int64_t>(out->n) * (out->xtype == kValF64 ? 8 : 4) <=
+                                     kClusterReplBytes
+                           : warp_slots <= kClusterWarpSlots;
+    if (CL.bytes <= kClusterSmem && pays) {
       out->cl_size = csize;
       out->cl_spc = spc;
       out->cl_slots = cap;
@@ -1346,7 +1476,7 @@ void SlicedMat::release(cudaStream_t s) {
   cl_size = cl_spc = cl_slots = 0;
   sten_w = 0;
   nslices = 0;
-  has_columns = false;
+  has_columns = direct = false;
 }
 
 SlicedView SlicedMat::view() const {
@@ -1361,6 +1491,7 @@ SlicedView SlicedMat::view() const {
   v.vtype = vtype;
   v.cap_slots = cap_slots;
   v.cols_staged = has_columns ? 1 : 0;
+  v.direct = direct ? 1 : 0;
   v.batch = batch;
   v.xtype = xtype;
   v.wait_ns = wait_ns;
@@ -1389,7 +1520,7 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
   BCMG_TRY(dev_alloc(&out->meta, ns, s));
   BCMG_TRY(width.alloc(ns, s));
   BCMG_TRY(kind.alloc(ns, s));
-  BCMG_TRY(stats.alloc(3, s));  // chunk max, any column slice, exact types
+  BCMG_TRY(stats.alloc(3, s));  // chunk max, column slots, exact types
   BCMG_TRY(tmp.alloc(scan_tmp_size(ns), s));
   const int blocks = ceil_div(ns, kWarpsPerBlock);
   launch(k_slice_shape, blocks, kWarpsPerBlock * 32, 0, s, n, ns, A.row, A.col, width.get(),
@@ -1432,6 +1563,12 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
   out->slots = slots;
   out->has_columns = h_stats[1] != 0;
   out->batch = static_cast<int32_t>((static_cast<int64_t>(slots) + ns - 1) / ns);
+  // k_sl_cols where most slots are column slots, except for 16-bit values in
+  // narrow slices, which the staged pipeline (32 consumer warps per SM at that
+  // size) streams a little faster: 1.2 M rows, 8.4 slots, BF16: 18.4 against
+  // 19.6 us per sweep; from 9.7 slots on the direct form is the faster one.
+  out->direct = h_stats[1] != 0 && 2 * static_cast<int64_t>(h_stats[1]) >= slots &&
+                !(value_bytes(vtype) == 2 && out->batch <= 9);
   const size_t vb = value_bytes(vtype);
   const int64_t padded = static_cast<int64_t>(slots) + kSlotPad;
   {
@@ -1492,7 +1629,7 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
   out->sten_w = 0;
   std::fill(out->sten_off, out->sten_off + kStencilMax, 0);
   if (const int kb = out->batch;
-      kb <= kStencilMax && kb <= 2 * slot_batch(out->batch, out->xtype == kValF64)) {
+      kb <= kStencilMax && kb <= 2 * slot_batch(out->batch, out->xtype == kValF64, out->direct)) {
     BCMG_CUDA(cudaMemcpyAsync(stats.get(), &ns, sizeof(int32_t), cudaMemcpyHostToDevice, s));
     launch(k_stencil_pick, ceil_div(ns, 256), 256, 0, s, ns, out->meta, kb, stats.get());
     BCMG_LAUNCH_CHECK();

@@ -78,6 +78,7 @@ struct SlicedView {
   int vtype = kValF64;
   int32_t cap_slots = 0;    // slots one pipeline stage holds
   int32_t cols_staged = 0;  // explicit columns exist (and are staged)
+  int32_t direct = 0;       // most slots are column slots: row passes by k_sl_cols
   int32_t batch = 0;        // mean slice width (chooses the slot batch size)
   int xtype = kValF64;      // vector type the copy serves (kValF64 or kValF32)
   unsigned long long wait_ns = kDefaultWaitNs;  // bound on each pipeline wait
@@ -102,6 +103,7 @@ struct SlicedMat {
   int xtype = kValF64;       // vector type served: kValF64 or kValF32
   bool narrowed = false;     // values stored narrower than xtype (all exact)
   bool has_columns = false;  // scol allocated (some slice is a column slice)
+  bool direct = false;       // see SlicedView
   unsigned long long wait_ns = kDefaultWaitNs;  // copied into every view
   int32_t cl_size = 0, cl_spc = 0, cl_slots = 0;  // see SlicedView
   int32_t sten_w = 0, sten_off[kStencilMax] = {};  // see SlicedView
