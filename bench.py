@@ -533,11 +533,14 @@ def run_ours(args):
     h.close()
     sweep_s = r0.elapsed_time(r1) / 1e3 / sweeps
     if vbytes.value:
-        # sliced copy: values incl. padding, explicit columns, per-slice
-        # metadata, and u (gathered once), f, d read + u' written
+        # sliced copy: values incl. padding (none in constant-coefficient
+        # slices), explicit columns, per-slice metadata, and u (gathered
+        # once), f, d read + u' written
         sweep_bytes = (vbytes.value * 32 * slots.value + 4 * 32 * cslots.value +
                        16 * nsl.value + 4 * xbytes * A.n)
-        kname = "k_sl_pipe<EpiRelax> (level-0 l1-Jacobi sweep, sliced, pipelined)"
+        kname = ("k_sl_uniform<EpiRelax> (level-0 l1-Jacobi sweep, constant stencil)"
+                 if 4 * slots.value < nsl.value else
+                 "k_sl_pipe or k_sl_cols<EpiRelax> (level-0 l1-Jacobi sweep, sliced copy)")
     else:
         sweep_bytes = 12 * A.nnz + 4 * (A.n + 1) + 36 * A.n
         kname = "k_relax_t (level-0 l1-Jacobi sweep, CSR)"

@@ -126,34 +126,178 @@ __global__ void k_slice_shape(int32_t n, int32_t nslices, const int32_t *__restr
   }
 }
 
-// Format statistics from the scanned slot pointers: stats[0] = the most slots
-// in one chunk of kPipeWarps slices, stats[1] = the slots of column slices.
+// The copy's stencil: the offsets of its first interior slice exactly as wide
+// as the mean slice, and one value per offset.
+struct Stencil {
+  int32_t w;
+  int32_t off[kStencilMax];
+  double val[kStencilMax];
+};
+enum { kStatChunk = 0, kStatColSlots, kStatExact, kStatFirst, kStatUniform, kStatUniformSlots,
+       kNumStats };
+// A copy is uniform when three quarters of its slices are (host and device).
+__host__ __device__ inline bool mostly_uniform(int32_t uniform, int32_t nslices) {
+  return 4 * static_cast<int64_t>(uniform) >= 3 * static_cast<int64_t>(nslices);
+}
+
+// Format statistics from the scanned slot pointers: the most slots in one
+// chunk of kPipeWarps slices, and the slots of column slices.
 __global__ void k_slice_stats(int32_t nslices, const int32_t *__restrict__ sptr,
                               const int32_t *__restrict__ kind, int32_t *stats) {
   const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   const int32_t s0 = c * kPipeWarps;
   if (s0 >= nslices) return;
   const int32_t s1 = min(s0 + kPipeWarps, nslices);
-  atomicMax(stats, sptr[s1] - sptr[s0]);
+  atomicMax(stats + kStatChunk, sptr[s1] - sptr[s0]);
   int32_t col_slots = 0;
   for (int32_t s = s0; s < s1; ++s)
     if (!kind[s]) col_slots += sptr[s + 1] - sptr[s];
-  if (col_slots) atomicAdd(stats + 1, col_slots);
+  if (col_slots) atomicAdd(stats + kStatColSlots, col_slots);
+}
+
+// Every row r of the slice is below n and r + o stays in [0, n) for every
+// offset o in [lo, hi].
+__device__ __forceinline__ bool slice_interior(int32_t n, int32_t s, int32_t lo, int32_t hi) {
+  const int64_t r0 = static_cast<int64_t>(s) * 32, r1 = r0 + 31;
+  return r1 < n && r0 + lo >= 0 && r1 + hi < n;
+}
+
+// The first interior offset slice as wide as the mean slice (none:
+// stats[kStatFirst] stays nslices).
+__global__ void k_stencil_find(int32_t n, int32_t nslices, const int32_t *__restrict__ sptr,
+                               const int32_t *__restrict__ width,
+                               const int32_t *__restrict__ kind,
+                               const int32_t *__restrict__ offrange, int32_t *stats) {
+  const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t w = (static_cast<int64_t>(sptr[nslices]) + nslices - 1) / nslices;
+  const bool hit = s < nslices && w <= kStencilMax && kind[s] == 1 && width[s] == w &&
+                   slice_interior(n, s, offrange[0], offrange[1]);
+  const unsigned lo = __reduce_min_sync(0xffffffffu, hit ? static_cast<unsigned>(s) : ~0u);
+  if ((threadIdx.x & 31) == 0 && lo != ~0u) atomicMin(stats + kStatFirst, static_cast<int32_t>(lo));
+}
+
+// One warp: the stencil of slice stats[kStatFirst] (values: those of the
+// first row that has the offset).
+__global__ void k_stencil_load(int32_t nslices, const int32_t *__restrict__ row,
+                               const int32_t *__restrict__ col, const double *__restrict__ val,
+                               const int32_t *__restrict__ width, const int32_t *stats,
+                               Stencil *st) {
+  const int lane = threadIdx.x;
+  const int32_t s = stats[kStatFirst];
+  if (s >= nslices) return;
+  const int32_t r = s * 32 + lane, w = width[s];
+  int32_t pos = row[r];
+  const int32_t e = row[r + 1];
+  for (int32_t k = 0; k < w; ++k) {
+    const int32_t cur = pos < e ? col[pos] - r : INT_MAX;
+    const int32_t m = __reduce_min_sync(0xffffffffu, cur);
+    const unsigned have = __ballot_sync(0xffffffffu, cur == m);
+    if (lane == __ffs(have) - 1) {
+      st->off[k] = m;
+      st->val[k] = val[pos];
+    }
+    if (cur == m) ++pos;
+  }
+  if (lane == 0) st->w = w;
+}
+
+// Which slices are uniform: every entry of their rows lies at a stencil
+// offset and has that offset's value.  ukind: 0 no, else the meta kind;
+// rmask: the offsets each row has.
+__global__ void k_stencil_match(int32_t n, int32_t nslices, const int32_t *__restrict__ row,
+                                const int32_t *__restrict__ col,
+                                const double *__restrict__ val,
+                                const int32_t *__restrict__ width, const Stencil *__restrict__ st,
+                                uint32_t *rmask, int32_t *ukind, int32_t *stats) {
+  __shared__ Stencil sh;
+  __shared__ int32_t cnt[2];
+  for (int i = threadIdx.x; i < kStencilMax; i += blockDim.x) {
+    sh.off[i] = st->off[i];
+    sh.val[i] = st->val[i];
+  }
+  if (threadIdx.x == 0) {
+    sh.w = st->w;
+    cnt[0] = cnt[1] = 0;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int32_t s = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (s < nslices) {
+    const int32_t r = s * 32 + lane, w = sh.w;
+    int32_t pos = 0, e = 0;
+    if (r < n) {
+      pos = row[r];
+      e = row[r + 1];
+    }
+    bool ok = w > 0;
+    uint32_t mask = 0;
+    int32_t c = pos < e ? col[pos] - r : INT_MAX;
+    for (int32_t k = 0; k < w; ++k) {
+      if (c == sh.off[k]) {
+        ok = ok && val[pos] == sh.val[k];
+        mask |= 1u << k;
+        ++pos;
+        c = pos < e ? col[pos] - r : INT_MAX;
+      }
+      if (!__all_sync(0xffffffffu, ok)) break;
+    }
+    ok = __all_sync(0xffffffffu, ok && pos == e);
+    const bool full = __all_sync(0xffffffffu, w > 0 && mask == (~0u >> (32 - w)));
+    if (ok) rmask[r] = mask;
+    if (lane == 0) {
+      const bool in = ok && slice_interior(n, s, sh.off[0], sh.off[w - 1]);
+      ukind[s] = !ok ? 0 : (in ? (full ? 4 : 5) : 6);
+      if (ok) {
+        atomicAdd(&cnt[0], 1);
+        atomicAdd(&cnt[1], width[s]);
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && cnt[0]) {
+    atomicAdd(stats + kStatUniform, cnt[0]);
+    atomicAdd(stats + kStatUniformSlots, cnt[1]);
+  }
+}
+
+__device__ __forceinline__ int value_exact(double v) {
+  int ok = 7;
+  if (static_cast<double>(static_cast<float>(v)) != v) ok &= ~1;
+  if (static_cast<double>(__bfloat162float(__double2bfloat16(v))) != v) ok &= ~2;
+  if (static_cast<double>(__half2float(__double2half(v))) != v) ok &= ~4;
+  return ok;
 }
 
 // Which narrower types hold every value exactly (bitwise round trip):
-// bit 0 FP32, bit 1 BF16, bit 2 FP16; stats[2] starts at 7 and is and-ed.
-__global__ void k_value_exact(int64_t nnz, const double *__restrict__ val, int32_t *stats) {
+// bit 0 FP32, bit 1 BF16, bit 2 FP16; stats[kStatExact] starts at 7 and is
+// and-ed.  Uniform slices count through the stencil's values alone.
+__global__ void k_value_exact(int32_t n, int32_t nslices, int64_t nnz,
+                              const int32_t *__restrict__ row, const double *__restrict__ val,
+                              const int32_t *__restrict__ ukind, const Stencil *__restrict__ st,
+                              int32_t *stats) {
   int ok = 7;
-  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < nnz;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const double v = val[e];
-    if (static_cast<double>(static_cast<float>(v)) != v) ok &= ~1;
-    if (static_cast<double>(__bfloat162float(__double2bfloat16(v))) != v) ok &= ~2;
-    if (static_cast<double>(__half2float(__double2half(v))) != v) ok &= ~4;
+  const int lane = threadIdx.x & 31;
+  if (mostly_uniform(stats[kStatUniform], nslices)) {
+    if (blockIdx.x == 0 && threadIdx.x < st->w) ok &= value_exact(st->val[threadIdx.x]);
+    const int32_t warps = gridDim.x * blockDim.x / 32;
+    for (int32_t s = (blockIdx.x * blockDim.x + threadIdx.x) / 32; s < nslices; s += warps)
+      if (!ukind[s])
+        for (int32_t e = row[s * 32] + lane; e < row[min(s * 32 + 32, n)]; e += 32)
+          ok &= value_exact(val[e]);
+  } else {
+    for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < nnz;
+         e += static_cast<int64_t>(gridDim.x) * blockDim.x)
+      ok &= value_exact(val[e]);
   }
   ok = __reduce_and_sync(0xffffffffu, ok);
-  if ((threadIdx.x & 31) == 0 && ok != 7) atomicAnd(stats + 2, ok);
+  if (lane == 0 && ok != 7) atomicAnd(stats + kStatExact, ok);
+}
+
+// Uniform slices store no slots.
+__global__ void k_drop_uniform(int32_t nslices, const int32_t *__restrict__ ukind,
+                               int32_t *width) {
+  const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < nslices && ukind[s]) width[s] = 0;
 }
 
 // Pass 2: fill values (and columns or offsets).
@@ -231,10 +375,12 @@ __global__ void k_slice_heads(int32_t nslices, const int32_t *__restrict__ flag,
 // row r of the slice is below n and r + o stays in [0, n) for every offset o
 // in offrange, which bounds every entry of soff (offsets of offset slices,
 // zeros elsewhere), so its gathers need no clamping; 3 (k_slice_stencil) an
-// interior slice whose offsets are the copy's stencil.
+// interior slice whose offsets are the copy's stencil; 4 to 6 the uniform
+// slices of a uniform copy (ukind; null otherwise).
 __global__ void k_slice_meta(int32_t n, int32_t nslices, const int32_t *__restrict__ sptr,
                              const int32_t *__restrict__ width,
                              const int32_t *__restrict__ kind,
+                             const int32_t *__restrict__ ukind,
                              const int32_t *__restrict__ flag,
                              const int32_t *__restrict__ rid,
                              const int32_t *__restrict__ head,
@@ -242,35 +388,20 @@ __global__ void k_slice_meta(int32_t n, int32_t nslices, const int32_t *__restri
   const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nslices) return;
   const int32_t h = head[rid[s] + flag[s] - 1];
-  const int64_t r0 = static_cast<int64_t>(s) * 32, r1 = r0 + 31;
-  const bool interior =
-      kind[s] == 1 && r1 < n && r0 + offrange[0] >= 0 && r1 + offrange[1] < n;
-  meta[s] = make_int4(sptr[s], width[s], interior ? 2 : kind[s], sptr[h]);
+  const bool interior = kind[s] == 1 && slice_interior(n, s, offrange[0], offrange[1]);
+  const int32_t u = ukind ? ukind[s] : 0;
+  meta[s] = make_int4(sptr[s], width[s], u ? u : (interior ? 2 : kind[s]), sptr[h]);
 }
 
-// The first interior slice exactly w slots wide (none: *first stays nslices).
-__global__ void k_stencil_pick(int32_t nslices, const int4 *__restrict__ meta, int32_t w,
-                               int32_t *first) {
-  const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  bool hit = false;
-  if (s < nslices) {
-    const int4 m = meta[s];
-    hit = m.z == 2 && m.y == w;
-  }
-  const unsigned lo = __reduce_min_sync(0xffffffffu, hit ? static_cast<unsigned>(s) : ~0u);
-  if ((threadIdx.x & 31) == 0 && lo != ~0u) atomicMin(first, static_cast<int32_t>(lo));
-}
-
-// Marks interior slices whose offset list is the stencil soff[base .. base +
-// w) (the list of one interior slice of width w) as kind 3.
+// Marks interior slices whose offset list is the stencil's as kind 3.
 __global__ void k_slice_stencil(int32_t nslices, const int32_t *__restrict__ soff,
-                                int32_t base, int32_t w, int4 *meta) {
+                                const Stencil *__restrict__ st, int4 *meta) {
   const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nslices) return;
   int4 m = meta[s];
-  if (m.z != 2 || m.y != w) return;
-  for (int32_t i = 0; i < w; ++i)
-    if (soff[m.w + i] != soff[base + i]) return;
+  if (m.z != 2 || m.y != st->w) return;
+  for (int32_t i = 0; i < m.y; ++i)
+    if (soff[m.w + i] != st->off[i]) return;
   m.z = 3;
   meta[s] = m;
 }
@@ -365,6 +496,14 @@ __device__ __forceinline__ double gather(const double *x, int32_t i) {
   return v;
 }
 
+// p, as a value the compiler first knows here: read-only loads through it
+// cannot move above a pdl_wait() that precedes this call.
+template <typename T>
+__device__ __forceinline__ const T *after_wait(const T *p) {
+  asm volatile("" : "+l"(p));
+  return p;
+}
+
 // Gathers of a row sum from the iterate in global memory: x[i], or x[r + o]
 // relative to the row set by row() (one 64-bit multiply-add per gather).
 template <typename XT>
@@ -374,9 +513,10 @@ struct GlobalGather {
   __device__ void row(int32_t r) { xr = x + r; }
   __device__ XT operator()(int32_t i) const { return gather(x, i); }
   __device__ XT rel(int32_t o) const { return gather(xr, o); }
-  // x[r + o] for an offset held in a kernel parameter: plain C, so the
-  // offset stays a constant-bank operand of the address arithmetic.
-  __device__ XT rel_param(int32_t o) const { return __ldg(xr + o); }
+  // x[r + o + d] for an offset o held in a kernel parameter and a constant d:
+  // plain C, so o stays a constant-bank operand of the address arithmetic and
+  // d an immediate of the load.
+  __device__ XT rel_param(int32_t o, int d = 0) const { return __ldg(xr + o + d); }
 };
 
 // One batch of KB slots of a slice row sum (see row_sum); Full: every slot
@@ -458,6 +598,79 @@ __device__ __forceinline__ XT stencil_row_sum(const VT *v, const SlicedView &S, 
 #pragma unroll
       for (int q = 0; q < K2; ++q)
         if (KB + q < W) t[q & 3] = fma(static_cast<XT>(widen(v[(KB + q) * 32])), xv[q], t[q & 3]);
+    }
+  }
+  return (t[0] + t[1]) + (t[2] + t[3]);
+}
+
+// Offsets and values of a uniform copy's stencil, kernel parameters (constant
+// bank operands of the address arithmetic and the multiply-adds).
+template <typename XT>
+struct UniformStencil {
+  int32_t w = 0;
+  int32_t off[kStencilMax] = {};
+  XT val[kStencilMax] = {};
+};
+template <typename XT>
+UniformStencil<XT> uniform_stencil(const SlicedView &S) {
+  UniformStencil<XT> u;
+  u.w = S.sten_w;
+  for (int k = 0; k < u.w; ++k) {
+    u.off[k] = S.sten_off[k];
+    u.val[k] = static_cast<XT>(S.sten_val[k]);
+  }
+  return u;
+}
+
+// Batch of a uniform copy's kernels (its other slices, the cluster): the
+// stencil's width where kernels are built for it, else 8.
+template <typename XT>
+constexpr int uniform_batch(int w) {
+  return w == 5 || w == 7 || (w == 27 && sizeof(XT) == 4) ? w : 8;
+}
+// The slot that starts slot k's run of consecutive offsets in the 5-, 7- and
+// 27-point stencils of a grid stored x-fastest (x - 1, x, x + 1).
+template <int W>
+constexpr int run_start(int k) {
+  if (W == 27) return k - k % 3;
+  if (W == 7 || W == 5) return k >= W / 2 - 1 && k <= W / 2 + 1 ? W / 2 - 1 : k;
+  return k;
+}
+
+// Row sum of a uniform slice's row; kind as meta.z, mask the offsets the row
+// has.  Slots in stencil order, four partial sums by slot index mod 4, missing
+// entries skipped: the order does not depend on the batch.  W: the stencil's
+// width where a kernel is built for it (its offsets then come in the runs of
+// run_start), 0: any.
+template <typename XT, int W, typename G>
+__device__ __forceinline__ XT uniform_row_sum(const UniformStencil<XT> &u, int kind,
+                                              uint32_t mask, int32_t r, int32_t hi, const G &g) {
+  constexpr int KB = W == 0 ? 8 : (W <= 14 ? W : (sizeof(XT) == 4 ? W : 9));
+  const int w = W ? W : u.w;
+  XT t[4] = {XT(0), XT(0), XT(0), XT(0)};
+#pragma unroll
+  for (int k = 0; k < (W ? W : kStencilMax); k += KB) {
+    if (!W && k >= w) break;
+    XT xv[KB];
+    if (kind != 6) {
+#pragma unroll
+      for (int q = 0; q < KB; ++q)
+        if (k + q < w)
+          xv[q] = g.rel_param(u.off[run_start<W>(k + q)], k + q - run_start<W>(k + q));
+    } else {
+#pragma unroll
+      for (int q = 0; q < KB; ++q)
+        if (k + q < w) xv[q] = g(min(max(r + u.off[k + q], 0), hi));
+    }
+    if (kind == 4) {
+#pragma unroll
+      for (int q = 0; q < KB; ++q)
+        if (k + q < w) t[(k + q) & 3] = fma(u.val[k + q], xv[q], t[(k + q) & 3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < KB; ++q)
+        if (k + q < w && (mask & (1u << (k + q))))
+          t[(k + q) & 3] = fma(u.val[k + q], xv[q], t[(k + q) & 3]);
     }
   }
   return (t[0] + t[1]) + (t[2] + t[3]);
@@ -620,7 +833,7 @@ constexpr int pipe_min_blocks() {
 // vectors and the gathers wait for that kernel.
 template <typename VT, typename XT, typename Epi, int KB>
 __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
-    k_sl_pipe(SlicedView S, const VT *__restrict__ val, const XT *__restrict__ x, Epi epi,
+    k_sl_pipe(SlicedView S, const VT *__restrict__ val, const XT *x, Epi epi,
               int cap_slots, int cols_staged) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kPipeStages], empty[kPipeStages];
@@ -731,6 +944,7 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
   // consumers
   if constexpr (!Epi::kGated) pdl_wait();
   pdl_trigger();
+  x = after_wait(x);
   const int32_t hi = S.n - 1;
   int32_t c = c_first;
   for (int j = 0; c < c_last; ++j, c += c_step) {
@@ -786,6 +1000,60 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
   epi.finish(wid, lane);
 }
 
+// ---- row passes of uniform copies -------------------------------------------
+// Constant-coefficient stencils: a uniform slice streams no values, only the
+// row vectors (and one mask word per row where some entry is missing), so
+// nothing is staged; a warp per slice gathers through L1, 27 (FP32 vectors)
+// or 9 (FP64) loads in flight per lane with 32 warps per SM.  27-point 128^3:
+// 33.5 MB instead of 146.7 per FP32 sweep; what bounds it now is instruction
+// issue (about 180 per 32 rows: a load, an address or half of one and a
+// multiply-add per slot, bit tests where entries are missing, the division).
+// Per sweep, against the staged pipeline with 16-bit values: level 0 31.3 ->
+// 18.0 us (FP32) and 39.2 -> 26.8 us (FP64), its 524 K-row level 9.3 -> 6.6
+// and 11.6 -> 8.5, 131 K rows 4.35 -> 2.7 and 5.4 -> 3.4.  Fewer loads in
+// flight with more warps in FP32 (9 or 14, 40 to 48 warps): 29 us.
+template <typename VT, typename XT, typename Epi, int W>
+__global__ void __launch_bounds__(kPipeWarps * 32, 4)
+    k_sl_uniform(SlicedView S, UniformStencil<XT> u, const VT *__restrict__ val,
+                 const XT *x, Epi epi) {
+  constexpr int NVS = Epi::NV > 0 ? Epi::NV : 1;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int32_t hi = S.n - 1, step = gridDim.x * kPipeWarps;
+  int32_t s = blockIdx.x * kPipeWarps + wid;
+  int4 m = __ldg(S.meta + min(s, S.nslices - 1));  // static: see k_sl_pipe
+  pdl_wait();
+  pdl_trigger();
+  x = after_wait(x);
+  if constexpr (Epi::kGated)
+    if (!epi.active()) return;
+  while (s < S.nslices) {
+    const int32_t r = s * 32 + lane;
+    const int4 mn = __ldg(S.meta + min(s + step, S.nslices - 1));
+    XT rv[NVS];
+#pragma unroll
+    for (int i = 0; i < NVS; ++i) rv[i] = XT(0);
+    if (r < S.n) {
+#pragma unroll
+      for (int i = 0; i < Epi::NV; ++i) rv[i] = epi.row_vec(i)[r];
+    }
+    GlobalGather<XT> g{x, x};
+    g.row(r);
+    XT T;
+    if (m.z >= 4) {
+      const uint32_t mask = m.z == 4 ? ~0u : __ldg(S.rmask + r);
+      T = uniform_row_sum<XT, W>(u, m.z, mask, r, hi, g);
+    } else {
+      const int64_t at = static_cast<int64_t>(m.x) * 32 + lane;
+      T = row_sum<VT, XT, uniform_batch<XT>(W)>(val + at, m.z ? nullptr : S.scol + at,
+                                                S.soff + m.w, m.y, r, hi, m.z == 2, g);
+    }
+    if (r < S.n) epi.apply(r, T, rv);
+    s += step;
+    m = mn;
+  }
+  epi.finish(wid, lane);
+}
+
 // ---- row passes of column-slice copies ------------------------------------
 // Rows with unordered columns: a gather of the iterate touches up to 32
 // sectors, so a pass is bound by the gathers an SM keeps in flight and by
@@ -810,7 +1078,7 @@ constexpr int kColBatch = 12;  // gathers in flight per lane
 
 template <typename VT, typename XT, typename Epi>
 __global__ void __launch_bounds__(kPipeWarps * 32, sizeof(XT) == 8 ? 2 : 3)
-    k_sl_cols(SlicedView S, const VT *__restrict__ val, const XT *__restrict__ x, Epi epi) {
+    k_sl_cols(SlicedView S, const VT *__restrict__ val, const XT *x, Epi epi) {
   constexpr int NVS = Epi::NV > 0 ? Epi::NV : 1, KB = kColBatch;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int32_t hi = S.n - 1, step = gridDim.x * kPipeWarps;
@@ -826,6 +1094,7 @@ __global__ void __launch_bounds__(kPipeWarps * 32, sizeof(XT) == 8 ? 2 : 3)
   }
   pdl_wait();
   pdl_trigger();
+  x = after_wait(x);
   if constexpr (Epi::kGated)
     if (!epi.active()) return;
   while (s < S.nslices) {
@@ -967,9 +1236,9 @@ constexpr int64_t kClusterReplBytes = 24 * 1024;
 // a remote CTA's iterate sits where the local one does.  xslices: slices of
 // the iterate that a CTA holds (its own, or all of them when replicated).
 struct ClusterLayout {
-  uint32_t vals, cols, meta, x0, x1, f, d, bytes;
+  uint32_t vals, cols, meta, x0, x1, f, d, mask, bytes;
   __host__ __device__ ClusterLayout(int slots, int vbytes, bool cols_on, int spc, int xslices,
-                                    int xbytes) {
+                                    int xbytes, bool masks) {
     vals = 0;
     cols = vals + ((static_cast<uint32_t>(slots) * 32u * vbytes + 15u) & ~15u);
     meta = cols + (cols_on ? static_cast<uint32_t>(slots) * 32u * 4u : 0u);
@@ -979,7 +1248,8 @@ struct ClusterLayout {
     x1 = x0 + xrows;
     f = x1 + xrows;
     d = f + rows;
-    bytes = d + rows;
+    mask = d + rows;
+    bytes = mask + (masks ? static_cast<uint32_t>(spc) * 128u : 0u);
   }
 };
 
@@ -990,6 +1260,7 @@ struct ClusterArgs {
   XT *res;    // f - A u after the sweeps (nullptr: none)
   int k;      // sweeps
   int zero_start;
+  UniformStencil<XT> uni;  // of a uniform copy
 };
 
 // Gathers from the iterate distributed over the cluster's shared memory: row
@@ -1006,7 +1277,7 @@ struct DistributedGather {
     return base[j & mask];
   }
   __device__ XT rel(int32_t o) const { return (*this)(r + o); }
-  __device__ XT rel_param(int32_t o) const { return (*this)(r + o); }
+  __device__ XT rel_param(int32_t o, int d = 0) const { return (*this)(r + o + d); }
 };
 
 // Gathers from the CTA's own copy of the whole iterate.
@@ -1017,7 +1288,7 @@ struct ReplicatedGather {
   __device__ void row(int32_t r) { xr = x + r; }
   __device__ XT operator()(int32_t i) const { return x[i]; }
   __device__ XT rel(int32_t o) const { return xr[o]; }
-  __device__ XT rel_param(int32_t o) const { return xr[o]; }
+  __device__ XT rel_param(int32_t o, int d = 0) const { return xr[o + d]; }
 };
 
 // Shared-memory address of the same variable in CTA `rank` of the cluster,
@@ -1034,13 +1305,22 @@ __device__ __forceinline__ void cluster_store(uint32_t addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
 
-template <typename VT, typename XT, int KB, bool Repl>
+// Form of a level's cluster passes: the iterate distributed or replicated, or
+// (uniform copies) distributed with the uniform slices' row sums.
+enum { kClusterDistributed = 0, kClusterReplicated, kClusterUniform };
+inline int cluster_form(bool uniform, bool has_columns) {
+  return uniform ? kClusterUniform : (has_columns ? kClusterReplicated : kClusterDistributed);
+}
+
+template <typename VT, typename XT, int KB, int Form>
 __global__ void __launch_bounds__(kClusterThreads)
     k_sl_cluster(SlicedView S, ClusterArgs<XT> a) {
+  constexpr bool Repl = Form == kClusterReplicated, Uni = Form == kClusterUniform;
+  constexpr int kUniW = KB != 8 && KB == uniform_batch<XT>(KB) ? KB : 0;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(128) unsigned char smem[];
   const ClusterLayout L(S.cl_slots, sizeof(VT), S.cols_staged != 0, S.cl_spc,
-                        Repl ? S.nslices : S.cl_spc, sizeof(XT));
+                        Repl ? S.nslices : S.cl_spc, sizeof(XT), Uni);
   __shared__ __align__(8) uint64_t loaded;
   const int q = static_cast<int>(cl.block_rank()), nq = static_cast<int>(cl.num_blocks());
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1055,6 +1335,7 @@ __global__ void __launch_bounds__(kClusterThreads)
   int4 *sm = reinterpret_cast<int4 *>(smem + L.meta);
   XT *xb0 = reinterpret_cast<XT *>(smem + L.x0), *xb1 = reinterpret_cast<XT *>(smem + L.x1);
   XT *sf = reinterpret_cast<XT *>(smem + L.f), *sd = reinterpret_cast<XT *>(smem + L.d);
+  uint32_t *smask = reinterpret_cast<uint32_t *>(smem + L.mask);
   const VT *val = static_cast<const VT *>(S.val);
   const int32_t p0 = S.sptr[s0], p1 = S.sptr[s1];
   // The CTA's slots plus the padding a batch may read past its last slice
@@ -1074,6 +1355,9 @@ __global__ void __launch_bounds__(kClusterThreads)
     if (cbytes) bulk_load(sc, S.scol + static_cast<int64_t>(p0) * 32, cbytes, &loaded);
     bulk_load(sm, S.meta + s0, mbytes, &loaded);
   }
+  if (Uni)
+    for (int32_t i = tid; i < (s1 - s0) * 32; i += kClusterThreads)
+      smask[i] = __ldg(S.rmask + r0 + i);
   pdl_wait();
   pdl_trigger();
   // Before a remote store: every CTA of the cluster has started.  (The
@@ -1116,9 +1400,14 @@ __global__ void __launch_bounds__(kClusterThreads)
       const int32_t r = (s0 + ls) * 32 + lane;
       const int64_t rel = static_cast<int64_t>(m.x - p0) * 32 + lane;
       gath.row(r);
-      const XT T = m.z == 3 ? stencil_row_sum<VT, XT, KB>(sv + rel, S, gath)
-                            : row_sum<VT, XT, KB>(sv + rel, m.z ? nullptr : sc + rel,
-                                                  S.soff + m.w, m.y, r, hi, m.z == 2, gath);
+      XT T;
+      if (Uni && m.z >= 4)
+        T = uniform_row_sum<XT, kUniW>(a.uni, m.z, smask[ls * 32 + lane], r, hi, gath);
+      else if (!Uni && m.z == 3)
+        T = stencil_row_sum<VT, XT, KB>(sv + rel, S, gath);
+      else
+        T = row_sum<VT, XT, KB>(sv + rel, m.z ? nullptr : sc + rel, S.soff + m.w, m.y, r, hi,
+                                m.z == 2, gath);
       if (r < S.n) {
         const int32_t rl = r - r0, xi = r - x_first;
         if (resid) {
@@ -1193,8 +1482,8 @@ bcmg_status pipe_cfg(K kernel, int threads, size_t stage_bytes, int32_t nchunks,
 // gathers per batch (two batches cover a 27-point row), which keeps three
 // CTAs per SM in the register file.  The summation order depends on KB, so
 // every kernel reading a copy uses this rule.
-// Copies whose slots are mostly column slots run k_sl_cols; there any multiple
-// of four gives its order, and 8 suits the cluster's gathers from shared memory.
+// Copies that run k_sl_cols sum slots by index mod 4; any multiple of four
+// gives that order, and 8 suits the cluster's gathers from shared memory.
 inline int slot_batch(int32_t batch, bool f64, bool direct) {
   if (direct) return 8;
   if (batch <= 5) return 5;
@@ -1203,6 +1492,24 @@ inline int slot_batch(int32_t batch, bool f64, bool direct) {
   if (f64) return 14;
   if (batch <= 16) return 16;
   return batch <= 27 ? 27 : 28;
+}
+
+// The stencil width a uniform copy's kernels are built for (0: any width).
+inline int uniform_width(const SlicedView &S) {
+  const int w = S.sten_w;
+  if (w != 5 && w != 7 && w != 27) return 0;
+  for (int k = 0; k < w; ++k) {
+    const int b = w == 5 ? run_start<5>(k) : (w == 7 ? run_start<7>(k) : run_start<27>(k));
+    if (S.sten_off[k] != S.sten_off[b] + (k - b)) return 0;
+  }
+  return w;
+}
+
+// Batch of a copy's kernels.
+inline int copy_batch(const SlicedView &S, bool f64) {
+  if (S.uniform)
+    return f64 ? uniform_batch<double>(uniform_width(S)) : uniform_batch<float>(uniform_width(S));
+  return slot_batch(S.batch, f64, S.direct != 0);
 }
 
 inline int value_bytes(int vtype) {
@@ -1215,6 +1522,20 @@ bcmg_status pipe_launch(const SlicedView &S, const XT *x, const Epi &epi, cudaSt
   if (S.nslices <= 0) return BCMG_OK;
   const int32_t nchunks = ceil_div(S.nslices, kPipeWarps);
   PipeCfg cfg;
+  if (S.uniform) {
+    const int w = uniform_width(S);
+    auto kern = w == 5    ? k_sl_uniform<VT, XT, Epi, 5>
+                : w == 7  ? k_sl_uniform<VT, XT, Epi, 7>
+                : w == 27 ? k_sl_uniform<VT, XT, Epi, 27>
+                          : k_sl_uniform<VT, XT, Epi, 0>;
+    BCMG_TRY(pipe_cfg(kern, kPipeWarps * 32, 0, nchunks, &cfg, Epi::kPartials));
+    if (!warm_only) {
+      launch_pdl(kern, cfg.grid, kPipeWarps * 32, 0, st, S, uniform_stencil<XT>(S),
+                 static_cast<const VT *>(S.val), x, epi);
+      BCMG_LAUNCH_CHECK();
+    }
+    return BCMG_OK;
+  }
   if (S.direct) {
     auto kern = k_sl_cols<VT, XT, Epi>;
     BCMG_TRY(pipe_cfg(kern, kPipeWarps * 32, 0, nchunks, &cfg, Epi::kPartials));
@@ -1234,7 +1555,7 @@ bcmg_status pipe_launch(const SlicedView &S, const XT *x, const Epi &epi, cudaSt
       launch_pdl(kern, cfg.grid, kPipeThreads, cfg.smem, st, S, static_cast<const VT *>(S.val), \
              x, epi, S.cap_slots, S.cols_staged);                                           \
   } while (0)
-  switch (slot_batch(S.batch, sizeof(XT) == 8, S.direct != 0)) {
+  switch (copy_batch(S, sizeof(XT) == 8)) {
     case 5: BCMG_PIPE_KB(5); break;
     case 7: BCMG_PIPE_KB(7); break;
     case 8: BCMG_PIPE_KB(8); break;
@@ -1252,10 +1573,10 @@ bcmg_status pipe_launch(const SlicedView &S, const XT *x, const Epi &epi, cudaSt
 // gather batch chosen as pipe_launch chooses it (the partial sums depend on
 // it).  The shared-memory attribute is set on first use, which sliced_build
 // makes happen outside any stream capture.
-template <typename VT, typename XT, int KB, bool Repl>
+template <typename VT, typename XT, int KB, int Form>
 bcmg_status cluster_launch_as(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
                               bool warm_only) {
-  auto kern = k_sl_cluster<VT, XT, KB, Repl>;
+  auto kern = k_sl_cluster<VT, XT, KB, Form>;
   {
     static std::mutex mu;
     static bool attr_set = false;
@@ -1268,7 +1589,8 @@ bcmg_status cluster_launch_as(const SlicedView &S, const ClusterArgs<XT> &a, cud
   }
   if (warm_only) return BCMG_OK;
   const ClusterLayout L(S.cl_slots, sizeof(VT), S.cols_staged != 0, S.cl_spc,
-                        Repl ? S.nslices : S.cl_spc, sizeof(XT));
+                        Form == kClusterReplicated ? S.nslices : S.cl_spc, sizeof(XT),
+                        Form == kClusterUniform);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S.cl_size);
   cfg.blockDim = dim3(kClusterThreads);
@@ -1288,18 +1610,22 @@ bcmg_status cluster_launch_as(const SlicedView &S, const ClusterArgs<XT> &a, cud
   return BCMG_OK;
 }
 
-// Copies with column slices keep the iterate replicated (see above).
 template <typename VT, typename XT, int KB>
 bcmg_status cluster_launch_kb(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
                               bool warm_only) {
-  return S.cols_staged ? cluster_launch_as<VT, XT, KB, true>(S, a, st, warm_only)
-                       : cluster_launch_as<VT, XT, KB, false>(S, a, st, warm_only);
+  switch (cluster_form(S.uniform != 0, S.cols_staged != 0)) {
+    case kClusterDistributed:
+      return cluster_launch_as<VT, XT, KB, kClusterDistributed>(S, a, st, warm_only);
+    case kClusterReplicated:
+      return cluster_launch_as<VT, XT, KB, kClusterReplicated>(S, a, st, warm_only);
+    default: return cluster_launch_as<VT, XT, KB, kClusterUniform>(S, a, st, warm_only);
+  }
 }
 
 template <typename VT, typename XT>
 bcmg_status cluster_launch(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
                            bool warm_only = false) {
-  switch (slot_batch(S.batch, sizeof(XT) == 8, S.direct != 0)) {
+  switch (copy_batch(S, sizeof(XT) == 8)) {
     case 5: return cluster_launch_kb<VT, XT, 5>(S, a, st, warm_only);
     case 7: return cluster_launch_kb<VT, XT, 7>(S, a, st, warm_only);
     case 8: return cluster_launch_kb<VT, XT, 8>(S, a, st, warm_only);
@@ -1308,7 +1634,7 @@ bcmg_status cluster_launch(const SlicedView &S, const ClusterArgs<XT> &a, cudaSt
   if constexpr (sizeof(XT) == 8) {
     return cluster_launch_kb<VT, XT, 14>(S, a, st, warm_only);
   } else {
-    switch (slot_batch(S.batch, false, S.direct != 0)) {
+    switch (copy_batch(S, false)) {
       case 16: return cluster_launch_kb<VT, XT, 16>(S, a, st, warm_only);
       case 27: return cluster_launch_kb<VT, XT, 27>(S, a, st, warm_only);
       default: return cluster_launch_kb<VT, XT, 28>(S, a, st, warm_only);
@@ -1416,7 +1742,7 @@ bcmg_status plan_cluster(SlicedMat *out, cudaStream_t s) {
     BCMG_CUDA(cudaMemcpyAsync(h_sptr.data(), out->sptr, sizeof(int32_t) * (ns + 1),
                               cudaMemcpyDeviceToHost, s));
     BCMG_CUDA(cudaStreamSynchronize(s));
-    const bool repl = out->has_columns;
+    const bool repl = cluster_form(out->uniform, out->has_columns) == kClusterReplicated;
     int32_t spc = ceil_div(ns, kClusterMax);
     if (!repl) {  // a power of two: the owner of a row is a shift away
       spc = 1;
@@ -1429,13 +1755,14 @@ bcmg_status plan_cluster(SlicedMat *out, cudaStream_t s) {
       cap = std::max(cap, h_sptr[s1] - h_sptr[s0]);
       for (int32_t w = 0; w < kClusterWarps; ++w) {
         int32_t t = 0;
-        for (int32_t i = s0 + w; i < s1; i += kClusterWarps) t += h_sptr[i + 1] - h_sptr[i];
+        for (int32_t i = s0 + w; i < s1; i += kClusterWarps)
+          t += std::max(h_sptr[i + 1] - h_sptr[i], out->uniform ? out->sten_w : 0);
         warp_slots = std::max(warp_slots, t);
       }
     }
     cap += kSlotPad;
-    const ClusterLayout CL(cap, static_cast<int>(value_bytes(out->vtype)), repl, spc,
-                           repl ? ns : spc, out->xtype == kValF64 ? 8 : 4);
+    const ClusterLayout CL(cap, static_cast<int>(value_bytes(out->vtype)), out->has_columns, spc,
+                           repl ? ns : spc, out->xtype == kValF64 ? 8 : 4, out->uniform);
     const bool pays = repl ? warp_slots <= kClusterWarpSlotsRepl &&
                                  static_cast<int64_t>(out->n) * (out->xtype == kValF64 ? 8 : 4) <=
                                      kClusterReplBytes
@@ -1449,6 +1776,16 @@ bcmg_status plan_cluster(SlicedMat *out, cudaStream_t s) {
   return BCMG_OK;
 }
 
+// A value as a copy stores it (narrow() on the host).
+double stored_value(double v, int vtype) {
+  switch (vtype) {
+    case kValF64: return v;
+    case kValF32: return static_cast<float>(v);
+    case kValBF16: return __bfloat162float(__double2bfloat16(v));
+    default: return __half2float(__double2half(v));
+  }
+}
+
 }  // namespace
 
 size_t SlicedMat::bytes() const {
@@ -1456,13 +1793,15 @@ size_t SlicedMat::bytes() const {
   const size_t vb = value_bytes(vtype);
   const size_t sl = (static_cast<size_t>(slots) + kSlotPad) * 32;
   return vb * sl + (has_columns ? 4 * sl : 0) + 4 * (static_cast<size_t>(slots) + kSlotPad) +
-         4 * (static_cast<size_t>(nslices) + 1) + 16 * static_cast<size_t>(nslices);
+         4 * (static_cast<size_t>(nslices) + 1) + 16 * static_cast<size_t>(nslices) +
+         (rmask ? 128 * static_cast<size_t>(nslices) : 0);
 }
 
 void SlicedMat::release(cudaStream_t s) {
   if (borrowed) {  // another copy owns the arrays
     sptr = scol = soff = nullptr;
     meta = nullptr;
+    rmask = nullptr;
     val = nullptr;
     borrowed = false;
   }
@@ -1470,13 +1809,14 @@ void SlicedMat::release(cudaStream_t s) {
   dev_free(meta, s);
   dev_free(scol, s);
   dev_free(soff, s);
+  dev_free(rmask, s);
   char *vp = static_cast<char *>(val);
   dev_free(vp, s);
   val = nullptr;
   cl_size = cl_spc = cl_slots = 0;
   sten_w = 0;
   nslices = 0;
-  has_columns = direct = false;
+  has_columns = direct = uniform = false;
 }
 
 SlicedView SlicedMat::view() const {
@@ -1499,7 +1839,12 @@ SlicedView SlicedMat::view() const {
   v.cl_spc = cl_spc;
   v.cl_slots = cl_slots;
   v.sten_w = sten_w;
-  for (int i = 0; i < kStencilMax; ++i) v.sten_off[i] = sten_off[i];
+  v.uniform = uniform ? 1 : 0;
+  v.rmask = rmask;
+  for (int i = 0; i < kStencilMax; ++i) {
+    v.sten_off[i] = sten_off[i];
+    v.sten_val[i] = sten_val[i];
+  }
   return v;
 }
 
@@ -1513,47 +1858,61 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
   out->nslices = ns;
   out->xtype = vtype == kValF64 ? kValF64 : kValF32;
   out->vtype = vtype;
-  DevBuf<int32_t> width, kind, stats, tmp, offrange;
+  DevBuf<int32_t> width, kind, ukind, stats, tmp, offrange;
+  DevBuf<Stencil> sten;
   BCMG_TRY(offrange.alloc(2, s));
   BCMG_CUDA(cudaMemsetAsync(offrange.get(), 0, 2 * sizeof(int32_t), s));  // 0 in the range
   BCMG_TRY(dev_alloc(&out->sptr, ns + 1, s));
   BCMG_TRY(dev_alloc(&out->meta, ns, s));
+  BCMG_TRY(dev_alloc(&out->rmask, static_cast<int64_t>(ns) * 32, s));
   BCMG_TRY(width.alloc(ns, s));
   BCMG_TRY(kind.alloc(ns, s));
-  BCMG_TRY(stats.alloc(3, s));  // chunk max, column slots, exact types
+  BCMG_TRY(ukind.alloc(ns, s));
+  BCMG_TRY(sten.alloc(1, s));
+  BCMG_TRY(stats.alloc(kNumStats, s));
   BCMG_TRY(tmp.alloc(scan_tmp_size(ns), s));
   const int blocks = ceil_div(ns, kWarpsPerBlock);
   launch(k_slice_shape, blocks, kWarpsPerBlock * 32, 0, s, n, ns, A.row, A.col, width.get(),
          kind.get(), offrange.get());
   BCMG_TRY(exclusive_scan(width.get(), out->sptr, ns, out->sptr + ns, tmp.get(), s));
-  BCMG_CUDA(cudaMemsetAsync(stats.get(), 0, 2 * sizeof(int32_t), s));
+  BCMG_CUDA(cudaMemsetAsync(sten.get(), 0, sizeof(Stencil), s));
+  {
+    int32_t init[kNumStats] = {};
+    init[kStatExact] = 7;
+    init[kStatFirst] = ns;
+    BCMG_CUDA(cudaMemcpyAsync(stats.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
+  }
+  const int32_t nchunks = ceil_div(ns, kPipeWarps);
+  launch(k_slice_stats, ceil_div(nchunks, 256), 256, 0, s, ns, out->sptr, kind.get(),
+         stats.get());
+  launch(k_stencil_find, ceil_div(ns, 256), 256, 0, s, n, ns, out->sptr, width.get(),
+         kind.get(), offrange.get(), stats.get());
+  launch(k_stencil_load, 1, 32, 0, s, ns, A.row, A.col, A.val, width.get(), stats.get(),
+         sten.get());
+  launch(k_stencil_match, blocks, kWarpsPerBlock * 32, 0, s, n, ns, A.row, A.col, A.val,
+         width.get(), sten.get(), out->rmask, ukind.get(), stats.get());
   // FP64 -> BF16 cuts the value stream 4x, FP32 -> BF16 2x; a copy serving
   // FP32 vectors narrows to BF16 or FP16 only, and copies already stored in
   // 16 bits (rounded on purpose) stay as they are.
   const bool try_narrow = narrow && (vtype == kValF64 || vtype == kValF32) && A.nnz > 0;
-  {
-    const int32_t all = 7;
-    BCMG_CUDA(cudaMemcpyAsync(stats.get() + 2, &all, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-  }
   if (try_narrow)
-    launch(k_value_exact, std::min<int64_t>(ceil_div(A.nnz, 256), 8 * kNumSM), 256, 0, s,
-           static_cast<int64_t>(A.nnz), A.val, stats.get());
-  const int32_t nchunks = ceil_div(ns, kPipeWarps);
-  launch(k_slice_stats, ceil_div(nchunks, 256), 256, 0, s, ns, out->sptr, kind.get(),
-         stats.get());
+    launch(k_value_exact, std::min<int64_t>(ceil_div(A.nnz, 256), 8 * kNumSM), 256, 0, s, n, ns,
+           static_cast<int64_t>(A.nnz), A.row, A.val, ukind.get(), sten.get(), stats.get());
   BCMG_LAUNCH_CHECK();
-  int32_t h_stats[4] = {0, 0, 0, 0};
-  BCMG_CUDA(cudaMemcpyAsync(h_stats, stats.get(), 3 * sizeof(int32_t), cudaMemcpyDeviceToHost,
+  int32_t h_stats[kNumStats] = {}, all_slots = 0;
+  Stencil h_sten = {};
+  BCMG_CUDA(cudaMemcpyAsync(h_stats, stats.get(), sizeof(h_stats), cudaMemcpyDeviceToHost, s));
+  BCMG_CUDA(cudaMemcpyAsync(&all_slots, out->sptr + ns, sizeof(int32_t), cudaMemcpyDeviceToHost,
                             s));
-  BCMG_CUDA(cudaMemcpyAsync(h_stats + 3, out->sptr + ns, sizeof(int32_t),
-                            cudaMemcpyDeviceToHost, s));
+  BCMG_CUDA(cudaMemcpyAsync(&h_sten, sten.get(), sizeof(Stencil), cudaMemcpyDeviceToHost, s));
   BCMG_CUDA(cudaStreamSynchronize(s));
-  const int32_t slots = h_stats[3];
+  out->uniform = h_sten.w > 0 && mostly_uniform(h_stats[kStatUniform], ns);
+  const int32_t slots = all_slots - (out->uniform ? h_stats[kStatUniformSlots] : 0);
   // Exact narrowing: the narrowest storage that holds every value bit for bit
   // (BF16, then FP16, then FP32); the kernels widen and accumulate in the
   // vector type, so the arithmetic is unchanged.
   if (try_narrow) {
-    const int exact = h_stats[2];
+    const int exact = h_stats[kStatExact];
     if (exact & 2) vtype = kValBF16;
     else if (exact & 4) vtype = kValF16;
     else if ((exact & 1) && vtype == kValF64) vtype = kValF32;
@@ -1561,14 +1920,21 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
   out->vtype = vtype;
   out->narrowed = out->vtype != (out->xtype == kValF64 ? kValF64 : kValF32);
   out->slots = slots;
-  out->has_columns = h_stats[1] != 0;
-  out->batch = static_cast<int32_t>((static_cast<int64_t>(slots) + ns - 1) / ns);
+  out->has_columns = h_stats[kStatColSlots] != 0;
+  out->batch = static_cast<int32_t>((static_cast<int64_t>(all_slots) + ns - 1) / ns);
   // k_sl_cols where most slots are column slots, except for 16-bit values in
   // narrow slices, which the staged pipeline (32 consumer warps per SM at that
   // size) streams a little faster: 1.2 M rows, 8.4 slots, BF16: 18.4 against
   // 19.6 us per sweep; from 9.7 slots on the direct form is the faster one.
-  out->direct = h_stats[1] != 0 && 2 * static_cast<int64_t>(h_stats[1]) >= slots &&
+  out->direct = !out->uniform && out->has_columns &&
+                2 * static_cast<int64_t>(h_stats[kStatColSlots]) >= slots &&
                 !(value_bytes(vtype) == 2 && out->batch <= 9);
+  if (out->uniform) {
+    launch(k_drop_uniform, ceil_div(ns, 256), 256, 0, s, ns, ukind.get(), width.get());
+    BCMG_TRY(exclusive_scan(width.get(), out->sptr, ns, out->sptr + ns, tmp.get(), s));
+  } else {
+    dev_free(out->rmask, s);
+  }
   const size_t vb = value_bytes(vtype);
   const int64_t padded = static_cast<int64_t>(slots) + kSlotPad;
   {
@@ -1620,35 +1986,25 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
     BCMG_TRY(exclusive_scan(flag.get(), rid.get(), ns, rid.get() + ns, tmp.get(), s));
     launch(k_slice_heads, ceil_div(ns, 256), 256, 0, s, ns, flag.get(), rid.get(), head.get());
     launch(k_slice_meta, ceil_div(ns, 256), 256, 0, s, n, ns, out->sptr, width.get(),
-           kind.get(), flag.get(), rid.get(), head.get(), offrange.get(), out->meta);
+           kind.get(), out->uniform ? ukind.get() : nullptr, flag.get(), rid.get(), head.get(),
+           offrange.get(), out->meta);
     BCMG_LAUNCH_CHECK();
   }
   // Stencil: the offsets of the first interior slice as wide as the mean
-  // slice width (at most two slot batches and kStencilMax) become kernel
-  // parameters for every slice that has the same list (kind 3).
+  // slice (at most two slot batches and kStencilMax) become kernel
+  // parameters for every slice that has the same list (kind 3), or, with
+  // their values, for the uniform slices.
   out->sten_w = 0;
   std::fill(out->sten_off, out->sten_off + kStencilMax, 0);
-  if (const int kb = out->batch;
-      kb <= kStencilMax && kb <= 2 * slot_batch(out->batch, out->xtype == kValF64, out->direct)) {
-    BCMG_CUDA(cudaMemcpyAsync(stats.get(), &ns, sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    launch(k_stencil_pick, ceil_div(ns, 256), 256, 0, s, ns, out->meta, kb, stats.get());
-    BCMG_LAUNCH_CHECK();
-    int32_t first = ns;
-    BCMG_CUDA(cudaMemcpyAsync(&first, stats.get(), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    BCMG_CUDA(cudaStreamSynchronize(s));
-    int4 hm = make_int4(0, 0, 0, 0);
-    if (first < ns) {
-      BCMG_CUDA(cudaMemcpyAsync(&hm, out->meta + first, sizeof(int4), cudaMemcpyDeviceToHost,
-                                s));
-      BCMG_CUDA(cudaStreamSynchronize(s));
-    }
-    if (first < ns && hm.z == 2 && hm.y == kb) {
-      BCMG_CUDA(cudaMemcpyAsync(out->sten_off, out->soff + hm.w, sizeof(int32_t) * kb,
-                                cudaMemcpyDeviceToHost, s));
-      launch(k_slice_stencil, ceil_div(ns, 256), 256, 0, s, ns, out->soff, hm.w, kb, out->meta);
+  if (h_sten.w > 0 &&
+      (out->uniform ||
+       h_sten.w <= 2 * slot_batch(out->batch, out->xtype == kValF64, out->direct))) {
+    out->sten_w = h_sten.w;
+    std::copy(h_sten.off, h_sten.off + h_sten.w, out->sten_off);
+    for (int k = 0; k < h_sten.w; ++k) out->sten_val[k] = stored_value(h_sten.val[k], vtype);
+    if (!out->uniform) {
+      launch(k_slice_stencil, ceil_div(ns, 256), 256, 0, s, ns, out->soff, sten.get(), out->meta);
       BCMG_LAUNCH_CHECK();
-      BCMG_CUDA(cudaStreamSynchronize(s));
-      out->sten_w = kb;
     }
   }
   // Stage capacity: the largest chunk, capped so two stages fit in shared
@@ -1657,7 +2013,7 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
   const size_t fixed = kPipeWarps * 16 + 3 * kPipeWarps * 32 * 8 + 128;
   const int32_t cap_max =
       static_cast<int32_t>((kMaxStageBytes - fixed) / per_slot) - kSlotPad;
-  out->cap_slots = std::max<int32_t>(1, std::min<int32_t>(h_stats[0], cap_max));
+  out->cap_slots = std::max<int32_t>(1, std::min<int32_t>(h_stats[kStatChunk], cap_max));
   BCMG_TRY(plan_cluster(out, s));
   BCMG_TRY(warm_kernels(out->view()));
   return BCMG_OK;
@@ -1798,6 +2154,7 @@ bcmg_status sliced_cluster(const SlicedView &S, const XT *d, const XT *f, XT *u,
   a.res = res;
   a.k = k;
   a.zero_start = zero_start ? 1 : 0;
+  if (S.uniform) a.uni = uniform_stencil<XT>(S);
   return cluster_dispatch<XT>(S, a, s, false);
 }
 template bcmg_status sliced_cluster<double>(const SlicedView &, const double *, const double *,

@@ -91,6 +91,14 @@ struct SlicedView {
   // the kernels take those offsets from their parameters.
   int32_t sten_w = 0;
   int32_t sten_off[kStencilMax] = {};
+  // Uniform copies (uniform != 0): most slices have one coefficient per
+  // stencil offset -- every entry at offset sten_off[k] equals sten_val[k] --
+  // and store no values, only one word per row, bit k set when the row has
+  // that entry (meta.z 4: interior, every bit set; 5: interior; 6: gathers
+  // clamped).
+  int32_t uniform = 0;
+  const uint32_t *rmask = nullptr;
+  double sten_val[kStencilMax] = {};
 };
 
 struct SlicedMat {
@@ -107,6 +115,9 @@ struct SlicedMat {
   unsigned long long wait_ns = kDefaultWaitNs;  // copied into every view
   int32_t cl_size = 0, cl_spc = 0, cl_slots = 0;  // see SlicedView
   int32_t sten_w = 0, sten_off[kStencilMax] = {};  // see SlicedView
+  bool uniform = false;                            // see SlicedView
+  uint32_t *rmask = nullptr;
+  double sten_val[kStencilMax] = {};
   bool borrowed = false;  // the arrays belong to another copy (sliced_alias)
   void release(cudaStream_t s);
   size_t bytes() const;  // device bytes held

@@ -358,7 +358,8 @@ bcmg_status bcmg_level_relax(bcmg_handle *h, int hrc, int level, const void *d_f
  * which solves from CSR): value slots (32 values each),
  * slots of slices with explicit columns (the rest share column offsets and
  * store no indices), slices, bytes per value (0: the level is solved from
- * CSR). */
+ * CSR).  Slices of a constant-coefficient stencil (one value per column
+ * offset throughout) store no slots. */
 bcmg_status bcmg_level_format(const bcmg_handle *h, int hrc, int level,
                               int64_t *slots, int64_t *column_slots,
                               int32_t *slices, int32_t *value_bytes);

@@ -1,7 +1,9 @@
 """Smoother sweeps of one level against a plain numpy sweep, at the edges of
 the row passes: column slices of every batch remainder, slices cut by the last
-row, offset slices inside a copy of column slices, and levels small enough
-for one thread-block cluster (distributed or replicated iterate).
+row, offset slices inside a copy of column slices, constant-coefficient
+stencils of the widths kernels are built for and of others, with and without
+missing entries, and levels small enough for one thread-block cluster
+(distributed or replicated iterate).
 
 One sweep (k = 1) runs the row pass, several run the cluster kernel where the
 level fits one.  Bound per row and sweep: a sum of m products in any order is
@@ -24,6 +26,18 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
+def constant_stencil(offsets, n, seed):
+    """One coefficient per offset, some entries left out at random: a uniform
+    copy whose rows have arbitrary masks."""
+    rng = np.random.default_rng(seed)
+    r = np.concatenate([np.arange(n - o) for o in offsets])
+    c = np.concatenate([np.arange(o, n) for o in offsets])
+    v = np.concatenate([np.full(n - o, -0.3 - 0.1 * k) for k, o in enumerate(offsets)])
+    keep = rng.uniform(size=r.size) < 0.97
+    S = sp.coo_matrix((v[keep], (r[keep], c[keep])), shape=(n, n)).tocsr()
+    return bc.CsrMatrix.from_scipy((S + S.T + sp.identity(n) * 9.7).tocsr())
+
+
 def banded_and_random(n):
     """A 5-point band on the first half of the rows, random columns on the rest."""
     g = random_sym_graph(n // 2, 9, seed=5, int_weights=False).to_scipy()
@@ -42,6 +56,12 @@ CASES = {
     "rgg_5003": lambda: wl.rgg(5003, seed=9),
     "poisson7_13x11x9": lambda: wl.poisson(7, 13, 11, 9),
     "poisson27_31": lambda: wl.poisson(27, 31, 31, 31),
+    "poisson27_70x33x5": lambda: wl.poisson(27, 70, 33, 5),
+    "poisson5_257x129": lambda: wl.poisson(5, 257, 129),
+    "const_w7_no_runs": lambda: constant_stencil([2, 5, 40], 9001, 1),
+    "const_w31": lambda: constant_stencil(list(range(1, 16)), 20011, 2),
+    "const_w27_no_runs": lambda: constant_stencil([1, 2, 3, 5, 8, 13, 21, 34, 55, 89, 144, 233,
+                                                   377], 30000, 3),
 }
 
 
