@@ -13,6 +13,13 @@
 // then gathers its V columns of x at every entry.  The matrix is therefore
 // read once per W right-hand sides, and each column's row sum is a
 // sequential FMA chain in CSR order, independent of V and of the block size.
+//
+// Kernels are launched programmatically (launch_pdl): each begins as the one
+// ahead drains and calls pdl_wait() before it reads that kernel's output.
+// They do not trigger the next one early: with several waves of blocks its
+// waiting blocks took the places of blocks still to run (7-point 96^3 x 32,
+// FP32 sweep: 107 us launched normally, 119 with an early trigger, 105
+// without; levels of 13 K rows 8.7 -> 6.9 us, smaller ones 4.7 -> 3.2).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -110,8 +117,7 @@ template <int V, int MODE, typename VT, typename XT>
 __global__ void __launch_bounds__(256)
     k_bt_rowop(int32_t n, int W, int lgL, const int32_t *__restrict__ row,
                const int32_t *__restrict__ col, const VT *__restrict__ val,
-               const XT *__restrict__ d, const XT *__restrict__ f, const XT *__restrict__ u,
-               XT *__restrict__ out) {
+               const XT *__restrict__ d, const XT *f, const XT *u, XT *__restrict__ out) {
   const int L = 1 << lgL;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t gi = t >> lgL;
@@ -124,6 +130,9 @@ __global__ void __launch_bounds__(256)
     j0 = row[i];
     len = row[i + 1] - j0;
   }
+  // (The matrix is not written by the kernel ahead: its row bounds need not
+  // wait for that kernel.)
+  pdl_wait();
   // The row's own f, u and d do not depend on the row sum: load them first.
   const int64_t o = static_cast<int64_t>(i) * W + static_cast<int64_t>(g) * V;
   Cols<XT, V> fv;
@@ -163,6 +172,7 @@ __global__ void __launch_bounds__(256)
 template <typename XT>
 __global__ void k_bt_relax_zero(int64_t total, int lgW, const XT *__restrict__ d,
                                 const XT *__restrict__ f, XT *__restrict__ out) {
+  pdl_wait();
   for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x)
     out[e] = f[e] / d[e >> lgW];
@@ -172,6 +182,7 @@ template <int V, typename XT>
 __global__ void k_bt_restrict(int32_t nc, int W, int lgL, const int32_t *__restrict__ rptr,
                               const int32_t *__restrict__ ridx, const XT *__restrict__ p,
                               const XT *__restrict__ x, XT *__restrict__ y) {
+  pdl_wait();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t I = t >> lgL;
   if (I >= nc) return;
@@ -196,6 +207,7 @@ template <int V, typename XT>
 __global__ void k_bt_prolong(int32_t n, int W, int lgL, const int32_t *__restrict__ agg,
                              const XT *__restrict__ p, const XT *__restrict__ xc,
                              XT *__restrict__ xf) {
+  pdl_wait();
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t i = t >> lgL;
   if (i >= n) return;
@@ -213,6 +225,7 @@ __global__ void k_bt_prolong(int32_t n, int W, int lgL, const int32_t *__restric
 // reads and the interleaved writes are contiguous.
 __global__ void k_bt_pack(int32_t n, int m, const double *__restrict__ src, int64_t ld,
                           double *__restrict__ dst, int W, int lgW) {
+  pdl_wait();
   __shared__ double tile[32][kBatchMax + 1];
   const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 32;
   const int r = threadIdx.x & 31;
@@ -230,6 +243,7 @@ __global__ void k_bt_pack(int32_t n, int m, const double *__restrict__ src, int6
 
 __global__ void k_bt_unpack(int32_t n, int m, const double *__restrict__ src, int W, int lgW,
                             double *__restrict__ dst, int64_t ld) {
+  pdl_wait();
   __shared__ double tile[32][kBatchMax + 1];
   const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 32;
   for (int e = threadIdx.x; e < 32 * W; e += blockDim.x) {
@@ -298,6 +312,7 @@ __device__ __forceinline__ double bt_reduce_col(const double *partials, int k, i
 __global__ void __launch_bounds__(kRedT)
     k_bt_dots(int64_t total, int W, const double *__restrict__ a, const double *__restrict__ b,
               const double *__restrict__ c, const double *__restrict__ d, double *partials) {
+  pdl_wait();
   double acc[2][1] = {{0.0}, {0.0}};
   for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -308,12 +323,14 @@ __global__ void __launch_bounds__(kRedT)
 }
 
 __global__ void k_bt_col_norms(const double *partials, int W, double *out) {
+  pdl_wait();
   const double s = bt_reduce_col(partials, 0, W, blockIdx.x);
   if (threadIdx.x == 0) out[blockIdx.x] = sqrt(s);
 }
 
 __global__ void k_bt_init(const double *partials, int W, double rtol, int itnlim,
                           double *scal) {
+  pdl_wait();
   const int c = blockIdx.x;
   const double rr = bt_reduce_col(partials, 0, W, c);
   const double bb = bt_reduce_col(partials, 1, W, c);
@@ -332,6 +349,7 @@ __global__ void k_bt_init(const double *partials, int W, double rtol, int itnlim
 }
 
 __global__ void k_bt_any_active(const double *scal, int W, int *flags) {
+  pdl_wait();
   const int c = threadIdx.x;
   const bool a = c < W && scal[c * kBtStride + kBtAct] != 0.0;
   const bool any = __any_sync(kFull, a);
@@ -346,6 +364,7 @@ __global__ void __launch_bounds__(kRedT)
                        const double *__restrict__ v, double *__restrict__ w,
                        const double *__restrict__ r, const double *__restrict__ q,
                        double *partials) {
+  pdl_wait();
   const int L = 1 << lgL;
   const int g = threadIdx.x & (L - 1);
   const int64_t groups = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> lgL;
@@ -395,6 +414,7 @@ __global__ void __launch_bounds__(kRedT)
 // arithmetic as the single-vector k_fcg_scalars; columns that stopped
 // iterating are left untouched.
 __global__ void k_bt_fcg_scalars(const double *partials, double *scal, int W, int first) {
+  pdl_wait();
   const int c = blockIdx.x;
   const double alpha = bt_reduce_col(partials, 0, W, c);
   const double beta = bt_reduce_col(partials, 1, W, c);
@@ -437,6 +457,7 @@ __global__ void __launch_bounds__(kRedT)
                     double *__restrict__ zp, const double *__restrict__ az,
                     double *__restrict__ azp, double *__restrict__ x, double *__restrict__ r,
                     const double *__restrict__ scal, double *partials) {
+  pdl_wait();
   double acc[1][1] = {{0.0}};
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const double *S = scal + (t0 & (W - 1)) * kBtStride;
@@ -463,6 +484,7 @@ __global__ void __launch_bounds__(kRedT)
 // kNorm = sqrt(sum) for active columns (key = kBtAct) or for columns that
 // replaced their residual (key = kReplace).
 __global__ void k_bt_norm_final(const double *partials, double *scal, int W, int key) {
+  pdl_wait();
   const int c = blockIdx.x;
   const double s = bt_reduce_col(partials, 0, W, c);
   if (threadIdx.x == 0 && scal[c * kBtStride + key] != 0.0) scal[c * kBtStride + kNorm] = sqrt(s);
@@ -471,6 +493,7 @@ __global__ void k_bt_norm_final(const double *partials, double *scal, int W, int
 // Residual replacement decision per column (k_replace_flag); flags[1] says
 // whether any column replaces.
 __global__ void k_bt_replace_flag(double *scal, int W, int every, int *flags) {
+  pdl_wait();
   const int c = threadIdx.x;
   bool due = false;
   if (c < W) {
@@ -493,6 +516,7 @@ __global__ void __launch_bounds__(kRedT)
                        const double *__restrict__ b, const double *__restrict__ x,
                        double *__restrict__ r, const double *__restrict__ scal,
                        const int *flags, double *partials) {
+  pdl_wait();
   if (flags[1] == 0) return;  // uniform over the grid
   const int L = 1 << lgL;
   const int g = threadIdx.x & (L - 1);
@@ -536,6 +560,7 @@ __global__ void __launch_bounds__(kRedT)
 // column still iterating".
 __global__ void k_bt_continue(double *scal, int W, int *flags, cudaGraphConditionalHandle cond,
                               int use_cond) {
+  pdl_wait();
   const int c = threadIdx.x;
   bool go = false;
   if (c < W) {
@@ -584,16 +609,16 @@ void launch_rowop_v(const MatView &A, int W, BtCfg cfg, const XT *d, const XT *f
   const int blocks = grid_of(static_cast<int64_t>(A.n) * L, cfg.threads);
   switch (cfg.V) {
     case 1:
-      launch(k_bt_rowop<1, MODE, VT, XT>, blocks, cfg.threads, 0, s, A.n, W, lgL, A.row,
+      launch_pdl(k_bt_rowop<1, MODE, VT, XT>, blocks, cfg.threads, 0, s, A.n, W, lgL, A.row,
              A.col, val, d, f, u, out);
       break;
     case 2:
-      launch(k_bt_rowop<2, MODE, VT, XT>, blocks, cfg.threads, 0, s, A.n, W, lgL, A.row,
+      launch_pdl(k_bt_rowop<2, MODE, VT, XT>, blocks, cfg.threads, 0, s, A.n, W, lgL, A.row,
              A.col, val, d, f, u, out);
       break;
     default:
       if constexpr (sizeof(XT) <= 4)
-        launch(k_bt_rowop<4, MODE, VT, XT>, blocks, cfg.threads, 0, s, A.n, W, lgL, A.row,
+        launch_pdl(k_bt_rowop<4, MODE, VT, XT>, blocks, cfg.threads, 0, s, A.n, W, lgL, A.row,
                A.col, val, d, f, u, out);
       break;
   }
@@ -641,10 +666,10 @@ bcmg_status bt_relax(const MatView &A, int W, BtCfg cfg, const XT *d, const XT *
   int left = k;
   if (zero_start) {
     cur = (k % 2 == 1) ? u : u_tmp;
-    launch(k_bt_relax_zero<XT>, stream_grid(total), 256, 0, s, total, ilog2(W), d, f, cur);
+    launch_pdl(k_bt_relax_zero<XT>, stream_grid(total), 256, 0, s, total, ilog2(W), d, f, cur);
     --left;
   } else if (k % 2 == 1) {
-    BCMG_CUDA(cudaMemcpyAsync(u_tmp, u, sizeof(XT) * total, cudaMemcpyDeviceToDevice, s));
+    BCMG_TRY(copy_t<XT>(u_tmp, u, total, s));  // a kernel: ordered before the first sweep
     cur = u_tmp;
   } else {
     cur = u;
@@ -678,11 +703,11 @@ bcmg_status bt_restrict(int32_t nc, const int32_t *rptr, const int32_t *ridx, co
   const int V = elem_v<XT>(W), L = W / V, lgL = ilog2(L);
   const int blocks = grid_of(static_cast<int64_t>(nc) * L, 256);
   switch (V) {
-    case 1: launch(k_bt_restrict<1, XT>, blocks, 256, 0, s, nc, W, lgL, rptr, ridx, p, x, y); break;
-    case 2: launch(k_bt_restrict<2, XT>, blocks, 256, 0, s, nc, W, lgL, rptr, ridx, p, x, y); break;
+    case 1: launch_pdl(k_bt_restrict<1, XT>, blocks, 256, 0, s, nc, W, lgL, rptr, ridx, p, x, y); break;
+    case 2: launch_pdl(k_bt_restrict<2, XT>, blocks, 256, 0, s, nc, W, lgL, rptr, ridx, p, x, y); break;
     default:
       if constexpr (sizeof(XT) <= 4)
-        launch(k_bt_restrict<4, XT>, blocks, 256, 0, s, nc, W, lgL, rptr, ridx, p, x, y);
+        launch_pdl(k_bt_restrict<4, XT>, blocks, 256, 0, s, nc, W, lgL, rptr, ridx, p, x, y);
       break;
   }
   BCMG_LAUNCH_CHECK();
@@ -696,11 +721,11 @@ bcmg_status bt_prolong(int32_t n, const int32_t *agg, const XT *p, const XT *xc,
   const int V = elem_v<XT>(W), L = W / V, lgL = ilog2(L);
   const int blocks = grid_of(static_cast<int64_t>(n) * L, 256);
   switch (V) {
-    case 1: launch(k_bt_prolong<1, XT>, blocks, 256, 0, s, n, W, lgL, agg, p, xc, xf); break;
-    case 2: launch(k_bt_prolong<2, XT>, blocks, 256, 0, s, n, W, lgL, agg, p, xc, xf); break;
+    case 1: launch_pdl(k_bt_prolong<1, XT>, blocks, 256, 0, s, n, W, lgL, agg, p, xc, xf); break;
+    case 2: launch_pdl(k_bt_prolong<2, XT>, blocks, 256, 0, s, n, W, lgL, agg, p, xc, xf); break;
     default:
       if constexpr (sizeof(XT) <= 4)
-        launch(k_bt_prolong<4, XT>, blocks, 256, 0, s, n, W, lgL, agg, p, xc, xf);
+        launch_pdl(k_bt_prolong<4, XT>, blocks, 256, 0, s, n, W, lgL, agg, p, xc, xf);
       break;
   }
   BCMG_LAUNCH_CHECK();
@@ -720,7 +745,7 @@ bcmg_status bt_unpack(int32_t n, int m, const double *src, int W, double *dst, i
                       cudaStream_t s) {
   if (n <= 0 || m <= 0) return BCMG_OK;
   if (m > W || ld < n) return set_error(BCMG_ERR_INTERNAL, "bad unpack shape");
-  launch(k_bt_unpack, ceil_div(n, 32), 256, 0, s, n, m, src, W, ilog2(W), dst, ld);
+  launch_pdl(k_bt_unpack, ceil_div(n, 32), 256, 0, s, n, m, src, W, ilog2(W), dst, ld);
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
@@ -729,9 +754,9 @@ bcmg_status bt_fcg_init(int32_t n, int W, const double *r, const double *b, doub
                         int itnlim, double *partials, double *scal, int *flags,
                         cudaStream_t s) {
   const int64_t total = static_cast<int64_t>(n) * W;
-  launch(k_bt_dots, kRedBlocks, kRedT, 0, s, total, W, r, r, b, b, partials);
-  launch(k_bt_init, W, kRedT, 0, s, partials, W, rtol, itnlim, scal);
-  launch(k_bt_any_active, 1, 32, 0, s, scal, W, flags);
+  launch_pdl(k_bt_dots, kRedBlocks, kRedT, 0, s, total, W, r, r, b, b, partials);
+  launch_pdl(k_bt_init, W, kRedT, 0, s, partials, W, rtol, itnlim, scal);
+  launch_pdl(k_bt_any_active, 1, 32, 0, s, scal, W, flags);
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
@@ -742,10 +767,10 @@ bcmg_status bt_fcg_spmv_dots(const CsrView &A, int W, BtCfg cfg, const double *v
   BCMG_TRY(check_cfg(W, cfg, sizeof(double)));
   const int lgL = ilog2(W / cfg.V);
   if (cfg.V == 1)
-    launch(k_bt_fcg_spmv_dots<1>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
+    launch_pdl(k_bt_fcg_spmv_dots<1>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
            v, w, r, q, partials);
   else
-    launch(k_bt_fcg_spmv_dots<2>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
+    launch_pdl(k_bt_fcg_spmv_dots<2>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
            v, w, r, q, partials);
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
@@ -753,7 +778,7 @@ bcmg_status bt_fcg_spmv_dots(const CsrView &A, int W, BtCfg cfg, const double *v
 
 bcmg_status bt_fcg_scalars(const double *partials, double *scal, int W, bool first,
                            cudaStream_t s) {
-  launch(k_bt_fcg_scalars, W, kRedT, 0, s, partials, scal, W, first ? 1 : 0);
+  launch_pdl(k_bt_fcg_scalars, W, kRedT, 0, s, partials, scal, W, first ? 1 : 0);
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
@@ -762,9 +787,9 @@ bcmg_status bt_fcg_update(int32_t n, int W, bool first, const double *z, double 
                           const double *az, double *azp, double *x, double *r,
                           double *partials, double *scal, cudaStream_t s) {
   const int64_t total = static_cast<int64_t>(n) * W;
-  launch(k_bt_fcg_update, kRedBlocks, kRedT, 0, s, total, W, first ? 1 : 0, z, zp, az, azp, x,
+  launch_pdl(k_bt_fcg_update, kRedBlocks, kRedT, 0, s, total, W, first ? 1 : 0, z, zp, az, azp, x,
          r, scal, partials);
-  launch(k_bt_norm_final, W, kRedT, 0, s, partials, scal, W, static_cast<int>(kBtAct));
+  launch_pdl(k_bt_norm_final, W, kRedT, 0, s, partials, scal, W, static_cast<int>(kBtAct));
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
@@ -773,22 +798,22 @@ bcmg_status bt_fcg_replace(const CsrView &A, int W, BtCfg cfg, const double *b,
                            const double *x, double *r, double *partials, double *scal,
                            int *flags, int every, cudaStream_t s) {
   BCMG_TRY(check_cfg(W, cfg, sizeof(double)));
-  launch(k_bt_replace_flag, 1, 32, 0, s, scal, W, every, flags);
+  launch_pdl(k_bt_replace_flag, 1, 32, 0, s, scal, W, every, flags);
   const int lgL = ilog2(W / cfg.V);
   if (cfg.V == 1)
-    launch(k_bt_true_residual<1>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
+    launch_pdl(k_bt_true_residual<1>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
            b, x, r, scal, flags, partials);
   else
-    launch(k_bt_true_residual<2>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
+    launch_pdl(k_bt_true_residual<2>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
            b, x, r, scal, flags, partials);
-  launch(k_bt_norm_final, W, kRedT, 0, s, partials, scal, W, static_cast<int>(kReplace));
+  launch_pdl(k_bt_norm_final, W, kRedT, 0, s, partials, scal, W, static_cast<int>(kReplace));
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
 
 bcmg_status bt_fcg_continue(double *scal, int W, int *flags, cudaGraphConditionalHandle cond,
                             bool use_cond, cudaStream_t s) {
-  launch(k_bt_continue, 1, 32, 0, s, scal, W, flags, cond, use_cond ? 1 : 0);
+  launch_pdl(k_bt_continue, 1, 32, 0, s, scal, W, flags, cond, use_cond ? 1 : 0);
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
@@ -796,8 +821,8 @@ bcmg_status bt_fcg_continue(double *scal, int W, int *flags, cudaGraphConditiona
 bcmg_status bt_col_norms(int32_t n, int W, const double *a, double *partials, double *out,
                          cudaStream_t s) {
   const int64_t total = static_cast<int64_t>(n) * W;
-  launch(k_bt_dots, kRedBlocks, kRedT, 0, s, total, W, a, a, nullptr, nullptr, partials);
-  launch(k_bt_col_norms, W, kRedT, 0, s, partials, W, out);
+  launch_pdl(k_bt_dots, kRedBlocks, kRedT, 0, s, total, W, a, a, nullptr, nullptr, partials);
+  launch_pdl(k_bt_col_norms, W, kRedT, 0, s, partials, W, out);
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
