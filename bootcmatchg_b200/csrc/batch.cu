@@ -392,19 +392,39 @@ bcmg_status bt_precond(bcmg_handle *h, BatchState &S, const double *rhs, double 
   return BCMG_OK;
 }
 
+// z = B r, w = A z with the dots, the scalars and the fused update of one FCG
+// step (the body of FCG.cu:464-495, or of the loop FCG.cu:497-565).  A
+// mixed-precision handle keeps z in FP32 (c32.out0) and has the update round
+// the new r into the next cycle's right-hand side (c32.in0, current on entry).
+bcmg_status bt_step(bcmg_handle *h, BatchState &S, bool first) {
+  cudaStream_t s = h->stream;
+  const CsrView A = h->A0.view();
+  const int W = S.W;
+  const double *q = first ? nullptr : S.q;
+  if (h->mixed) {
+    CycleBufs<float> &B = S.c32;
+    BCMG_TRY(bt_precond_t<float>(h, S, B, B.in0, B.out0, true));
+    BCMG_TRY(bt_fcg_spmv_dots<float>(A, W, S.fcg, B.out0, S.w, S.r, q, S.partials, s));
+    BCMG_TRY(bt_fcg_scalars(S.partials, S.scal, W, first, s));
+    return bt_fcg_update<float>(A.n, W, first, B.out0, S.d, S.w, S.q, S.x, S.r, B.in0,
+                                S.partials, S.scal, s);
+  }
+  BCMG_TRY(bt_precond_t<double>(h, S, S.c64, S.r, S.v, true));
+  BCMG_TRY(bt_fcg_spmv_dots<double>(A, W, S.fcg, S.v, S.w, S.r, q, S.partials, s));
+  BCMG_TRY(bt_fcg_scalars(S.partials, S.scal, W, first, s));
+  return bt_fcg_update<double>(A.n, W, first, S.v, S.d, S.w, S.q, S.x, S.r, nullptr, S.partials,
+                               S.scal, s);
+}
+
 // One FCG iteration for all columns (the do-while body of FCG.cu:497-565).
 bcmg_status bt_iteration(bcmg_handle *h, BatchState &S, cudaGraphConditionalHandle cond,
                          bool use_cond) {
   cudaStream_t s = h->stream;
-  const CsrView A = h->A0.view();
   const int W = S.W;
-  BCMG_TRY(bt_precond(h, S, S.r, S.v, true));
-  BCMG_TRY(bt_fcg_spmv_dots(A, W, S.fcg, S.v, S.w, S.r, S.q, S.partials, s));
-  BCMG_TRY(bt_fcg_scalars(S.partials, S.scal, W, false, s));
-  BCMG_TRY(bt_fcg_update(A.n, W, false, S.v, S.d, S.w, S.q, S.x, S.r, S.partials, S.scal, s));
+  BCMG_TRY(bt_step(h, S, false));
   if (h->ext.replace_every > 0)
-    BCMG_TRY(bt_fcg_replace(A, W, S.fcg, S.b, S.x, S.r, S.partials, S.scal, S.flags,
-                            h->ext.replace_every, s));
+    BCMG_TRY(bt_fcg_replace(h->A0.view(), W, S.fcg, S.b, S.x, S.r, h->mixed ? S.c32.in0 : nullptr,
+                            S.partials, S.scal, S.flags, h->ext.replace_every, s));
   BCMG_TRY(bt_fcg_continue(S.scal, W, S.flags, cond, use_cond, s));
   return BCMG_OK;
 }
@@ -423,10 +443,8 @@ bcmg_status bt_fcg(bcmg_handle *h, BatchState &S, int m, bcmg_solve_info *infos,
   BCMG_TRY(bt_fcg_init(n, W, S.r, S.b, h->prm.rtol, h->prm.itnlim, S.partials, S.scal, S.flags,
                        s));
   // First step (FCG.cu:464-495) for the active columns.
-  BCMG_TRY(bt_precond(h, S, S.r, S.v, true));
-  BCMG_TRY(bt_fcg_spmv_dots(A, W, S.fcg, S.v, S.w, S.r, nullptr, S.partials, s));
-  BCMG_TRY(bt_fcg_scalars(S.partials, S.scal, W, true, s));
-  BCMG_TRY(bt_fcg_update(n, W, true, S.v, S.d, S.w, S.q, S.x, S.r, S.partials, S.scal, s));
+  if (h->mixed) BCMG_TRY(convert_d2f(static_cast<int64_t>(n) * W, S.r, S.c32.in0, s));
+  BCMG_TRY(bt_step(h, S, true));
   const bool graphs = h->ext.use_graphs && h->stream != nullptr;
   if (graphs && !S.exec) {
     if (capture_while_loop(

@@ -62,17 +62,21 @@ bcmg_status bt_unpack(int32_t n, int m, const double *src, int W, double *dst, i
 bcmg_status bt_fcg_init(int32_t n, int W, const double *r, const double *b, double rtol,
                         int itnlim, double *partials, double *scal, int *flags, cudaStream_t s);
 // w = A v with per-column alpha = r.v, beta = w.v, gamma = q.v (q may be null).
-bcmg_status bt_fcg_spmv_dots(const CsrView &A, int W, BtCfg cfg, const double *v, double *w,
+// v (and z below): FP64, or the mixed-precision cycle's FP32 result, widened
+// as it is read.  r32 (or null): receives r in FP32 wherever r changes.
+template <typename ZT>
+bcmg_status bt_fcg_spmv_dots(const CsrView &A, int W, BtCfg cfg, const ZT *v, double *w,
                              const double *r, const double *q, double *partials,
                              cudaStream_t s);
 bcmg_status bt_fcg_scalars(const double *partials, double *scal, int W, bool first,
                            cudaStream_t s);
-bcmg_status bt_fcg_update(int32_t n, int W, bool first, const double *z, double *zp,
-                          const double *az, double *azp, double *x, double *r,
+template <typename ZT>
+bcmg_status bt_fcg_update(int32_t n, int W, bool first, const ZT *z, double *zp,
+                          const double *az, double *azp, double *x, double *r, float *r32,
                           double *partials, double *scal, cudaStream_t s);
 bcmg_status bt_fcg_replace(const CsrView &A, int W, BtCfg cfg, const double *b,
-                           const double *x, double *r, double *partials, double *scal,
-                           int *flags, int every, cudaStream_t s);
+                           const double *x, double *r, float *r32, double *partials,
+                           double *scal, int *flags, int every, cudaStream_t s);
 bcmg_status bt_fcg_continue(double *scal, int W, int *flags, cudaGraphConditionalHandle cond,
                             bool use_cond, cudaStream_t s);
 // out[c] = ||a[:, c]||_2 for the W columns.

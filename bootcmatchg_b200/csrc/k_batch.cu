@@ -65,11 +65,12 @@ __host__ __device__ inline int ilog2(int v) {
 
 // acc[v] = sum_j a_ij x[col_j, g V + v] for the group's row i (len entries
 // from j0; len = 0 for rows past the end).  All 32 lanes of the warp must
-// call it together: the loop bounds are warp-uniform.
-template <int V, typename VT, typename XT>
+// call it together: the loop bounds are warp-uniform.  x may be stored in a
+// narrower type (GT) than the sum; its values are widened.
+template <int V, typename VT, typename XT, typename GT = XT>
 __device__ __forceinline__ void bt_row_sum(const int32_t *__restrict__ col,
                                            const VT *__restrict__ val,
-                                           const XT *__restrict__ x, int W, int L, int g,
+                                           const GT *__restrict__ x, int W, int L, int g,
                                            int32_t j0, int len, XT (&acc)[V]) {
   const int maxlen = static_cast<int>(__reduce_max_sync(kFull, static_cast<unsigned>(len)));
   const int64_t cofs = static_cast<int64_t>(g) * V;
@@ -91,19 +92,20 @@ __device__ __forceinline__ void bt_row_sum(const int32_t *__restrict__ col,
         ck[u] = __shfl_sync(kFull, cj, k0 + u, L);
         vk[u] = __shfl_sync(kFull, vj, k0 + u, L);
       }
-      Cols<XT, V> xv[kUnroll];
+      Cols<GT, V> xv[kUnroll];
       // All kUnroll gathers are issued unconditionally, so they are in flight
       // together: an absent entry carries column 0 (a valid row) and its
       // product is dropped below.  Entry k0 + u exists for this row when it
       // lies inside both the chunk (kn entries) and the row.
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u)
-        xv[u] = ldc<XT, V>(x + static_cast<int64_t>(ck[u]) * W + cofs);
+        xv[u] = ldc<GT, V>(x + static_cast<int64_t>(ck[u]) * W + cofs);
 #pragma unroll
       for (int u = 0; u < kUnroll; ++u)
         if (k0 + u < kn && base + k0 + u < len) {
 #pragma unroll
-          for (int v = 0; v < V; ++v) acc[v] = fma(vk[u], xv[u].v[v], acc[v]);
+          for (int v = 0; v < V; ++v)
+            acc[v] = fma(vk[u], static_cast<XT>(xv[u].v[v]), acc[v]);
         }
     }
   }
@@ -356,12 +358,16 @@ __global__ void k_bt_any_active(const double *scal, int W, int *flags) {
   if (c == 0) flags[0] = any ? 1 : 0;
 }
 
-// w = A v fused with the per-column alpha = r.v, beta = w.v, gamma = q.v.
-template <int V>
+// w = A v fused with the per-column alpha = r.v, beta = w.v, gamma = q.v.  The
+// mixed-precision handle passes the cycle's FP32 result as it is (ZT float):
+// every product and sum is FP64 on its widened values.  Half the gathered
+// bytes of a widened copy, which is what bounds the pass (7-point 96^3 x 32:
+// 292 us on the FP64 copy).
+template <int V, typename ZT>
 __global__ void __launch_bounds__(kRedT)
     k_bt_fcg_spmv_dots(int32_t n, int W, int lgL, const int32_t *__restrict__ row,
                        const int32_t *__restrict__ col, const double *__restrict__ val,
-                       const double *__restrict__ v, double *__restrict__ w,
+                       const ZT *__restrict__ v, double *__restrict__ w,
                        const double *__restrict__ r, const double *__restrict__ q,
                        double *partials) {
   pdl_wait();
@@ -386,14 +392,17 @@ __global__ void __launch_bounds__(kRedT)
       len = row[i + 1] - j0;
     }
     double T[V];
-    bt_row_sum<V, double, double>(col, val, v, W, L, g, j0, len, T);
+    bt_row_sum<V, double, double, ZT>(col, val, v, W, L, g, j0, len, T);
     if (valid) {
       const int64_t o = static_cast<int64_t>(i) * W + static_cast<int64_t>(g) * V;
       Cols<double, V> tw;
 #pragma unroll
       for (int u = 0; u < V; ++u) tw.v[u] = T[u];
       stc<double, V>(w + o, tw);
-      const Cols<double, V> vv = ldc<double, V>(v + o);
+      const Cols<ZT, V> vz = ldc<ZT, V>(v + o);
+      Cols<double, V> vv;
+#pragma unroll
+      for (int u = 0; u < V; ++u) vv.v[u] = static_cast<double>(vz.v[u]);
       const Cols<double, V> rv = ldc<double, V>(r + o);
 #pragma unroll
       for (int u = 0; u < V; ++u) {
@@ -451,12 +460,15 @@ __global__ void k_bt_fcg_scalars(const double *partials, double *scal, int W, in
 
 // The fused FCG update of k_fcg_update per column; stopped columns keep x and
 // r.  The grid stride is a multiple of W, so a thread always serves the same
-// column.
+// column.  z may be FP32 (see k_bt_fcg_spmv_dots); r32 (or null) receives r
+// rounded to FP32, the next cycle's right-hand side.
+template <typename ZT>
 __global__ void __launch_bounds__(kRedT)
-    k_bt_fcg_update(int64_t total, int W, int first, const double *__restrict__ z,
+    k_bt_fcg_update(int64_t total, int W, int first, const ZT *__restrict__ z,
                     double *__restrict__ zp, const double *__restrict__ az,
                     double *__restrict__ azp, double *__restrict__ x, double *__restrict__ r,
-                    const double *__restrict__ scal, double *partials) {
+                    float *__restrict__ r32, const double *__restrict__ scal,
+                    double *partials) {
   pdl_wait();
   double acc[1][1] = {{0.0}};
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -465,7 +477,7 @@ __global__ void __launch_bounds__(kRedT)
     const double theta = S[kTheta];
     const double theta2 = first ? theta : S[kTheta2];
     for (int64_t e = t0; e < total; e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-      double zi = z[e], ai = az[e];
+      double zi = static_cast<double>(z[e]), ai = az[e];
       if (!first) {
         zi = fma(-theta, zp[e], zi);
         ai = fma(-theta, azp[e], ai);
@@ -475,6 +487,7 @@ __global__ void __launch_bounds__(kRedT)
       x[e] = fma(theta2, zi, x[e]);
       const double ri = fma(-theta2, ai, r[e]);
       r[e] = ri;
+      if (r32) r32[e] = static_cast<float>(ri);
       acc[0][0] = fma(ri, ri, acc[0][0]);
     }
   }
@@ -490,7 +503,7 @@ __global__ void k_bt_norm_final(const double *partials, double *scal, int W, int
   if (threadIdx.x == 0 && scal[c * kBtStride + key] != 0.0) scal[c * kBtStride + kNorm] = sqrt(s);
 }
 
-// Residual replacement decision per column (k_replace_flag); flags[1] says
+// Residual replacement decision per column (as k_fcg_update's); flags[1] says
 // whether any column replaces.
 __global__ void k_bt_replace_flag(double *scal, int W, int every, int *flags) {
   pdl_wait();
@@ -514,8 +527,8 @@ __global__ void __launch_bounds__(kRedT)
     k_bt_true_residual(int32_t n, int W, int lgL, const int32_t *__restrict__ row,
                        const int32_t *__restrict__ col, const double *__restrict__ val,
                        const double *__restrict__ b, const double *__restrict__ x,
-                       double *__restrict__ r, const double *__restrict__ scal,
-                       const int *flags, double *partials) {
+                       double *__restrict__ r, float *__restrict__ r32,
+                       const double *__restrict__ scal, const int *flags, double *partials) {
   pdl_wait();
   if (flags[1] == 0) return;  // uniform over the grid
   const int L = 1 << lgL;
@@ -548,6 +561,7 @@ __global__ void __launch_bounds__(kRedT)
         if (rep[u]) {
           const double ri = b[o + u] - T[u];
           r[o + u] = ri;
+          if (r32) r32[o + u] = static_cast<float>(ri);
           acc[0][u] = fma(ri, ri, acc[0][u]);
         }
     }
@@ -555,7 +569,7 @@ __global__ void __launch_bounds__(kRedT)
   bt_block_partials<1, V>(acc, W, L, partials);
 }
 
-// End of an iteration per column (k_fcg_continue): count it, stop the column
+// End of an iteration per column (fcg_end_iteration): count it, stop the column
 // when it converged, hit itnlim or broke down; the WHILE condition is "some
 // column still iterating".
 __global__ void k_bt_continue(double *scal, int W, int *flags, cudaGraphConditionalHandle cond,
@@ -761,17 +775,18 @@ bcmg_status bt_fcg_init(int32_t n, int W, const double *r, const double *b, doub
   return BCMG_OK;
 }
 
-bcmg_status bt_fcg_spmv_dots(const CsrView &A, int W, BtCfg cfg, const double *v, double *w,
+template <typename ZT>
+bcmg_status bt_fcg_spmv_dots(const CsrView &A, int W, BtCfg cfg, const ZT *v, double *w,
                              const double *r, const double *q, double *partials,
                              cudaStream_t s) {
   BCMG_TRY(check_cfg(W, cfg, sizeof(double)));
   const int lgL = ilog2(W / cfg.V);
   if (cfg.V == 1)
-    launch_pdl(k_bt_fcg_spmv_dots<1>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
-           v, w, r, q, partials);
+    launch_pdl(k_bt_fcg_spmv_dots<1, ZT>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col,
+               A.val, v, w, r, q, partials);
   else
-    launch_pdl(k_bt_fcg_spmv_dots<2>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
-           v, w, r, q, partials);
+    launch_pdl(k_bt_fcg_spmv_dots<2, ZT>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col,
+               A.val, v, w, r, q, partials);
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
@@ -783,29 +798,30 @@ bcmg_status bt_fcg_scalars(const double *partials, double *scal, int W, bool fir
   return BCMG_OK;
 }
 
-bcmg_status bt_fcg_update(int32_t n, int W, bool first, const double *z, double *zp,
-                          const double *az, double *azp, double *x, double *r,
+template <typename ZT>
+bcmg_status bt_fcg_update(int32_t n, int W, bool first, const ZT *z, double *zp,
+                          const double *az, double *azp, double *x, double *r, float *r32,
                           double *partials, double *scal, cudaStream_t s) {
   const int64_t total = static_cast<int64_t>(n) * W;
-  launch_pdl(k_bt_fcg_update, kRedBlocks, kRedT, 0, s, total, W, first ? 1 : 0, z, zp, az, azp, x,
-         r, scal, partials);
+  launch_pdl(k_bt_fcg_update<ZT>, kRedBlocks, kRedT, 0, s, total, W, first ? 1 : 0, z, zp, az,
+             azp, x, r, r32, scal, partials);
   launch_pdl(k_bt_norm_final, W, kRedT, 0, s, partials, scal, W, static_cast<int>(kBtAct));
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
 }
 
 bcmg_status bt_fcg_replace(const CsrView &A, int W, BtCfg cfg, const double *b,
-                           const double *x, double *r, double *partials, double *scal,
-                           int *flags, int every, cudaStream_t s) {
+                           const double *x, double *r, float *r32, double *partials,
+                           double *scal, int *flags, int every, cudaStream_t s) {
   BCMG_TRY(check_cfg(W, cfg, sizeof(double)));
   launch_pdl(k_bt_replace_flag, 1, 32, 0, s, scal, W, every, flags);
   const int lgL = ilog2(W / cfg.V);
   if (cfg.V == 1)
     launch_pdl(k_bt_true_residual<1>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
-           b, x, r, scal, flags, partials);
+           b, x, r, r32, scal, flags, partials);
   else
     launch_pdl(k_bt_true_residual<2>, kRedBlocks, kRedT, 0, s, A.n, W, lgL, A.row, A.col, A.val,
-           b, x, r, scal, flags, partials);
+           b, x, r, r32, scal, flags, partials);
   launch_pdl(k_bt_norm_final, W, kRedT, 0, s, partials, scal, W, static_cast<int>(kReplace));
   BCMG_LAUNCH_CHECK();
   return BCMG_OK;
@@ -840,5 +856,16 @@ bcmg_status bt_col_norms(int32_t n, int W, const double *a, double *partials, do
 
 BCMG_BT_INSTANTIATE(double)
 BCMG_BT_INSTANTIATE(float)
+
+#define BCMG_BT_FCG_INSTANTIATE(ZT)                                                          \
+  template bcmg_status bt_fcg_spmv_dots<ZT>(const CsrView &, int, BtCfg, const ZT *, double *, \
+                                            const double *, const double *, double *,          \
+                                            cudaStream_t);                                     \
+  template bcmg_status bt_fcg_update<ZT>(int32_t, int, bool, const ZT *, double *,             \
+                                         const double *, double *, double *, double *, float *, \
+                                         double *, double *, cudaStream_t);
+
+BCMG_BT_FCG_INSTANTIATE(double)
+BCMG_BT_FCG_INSTANTIATE(float)
 
 }  // namespace bcmg
