@@ -1198,10 +1198,10 @@ __global__ void k_wait_selftest(const int4 *__restrict__ src, unsigned long long
 // launch: CTA q loads slices [q spc, (q + 1) spc) -- values, explicit
 // columns, metadata, f and d -- once, with a cluster barrier between passes.
 // The iterate lives in shared memory in one of two ways:
-//   distributed (copies made of offset slices): a CTA holds its own rows and
+//   distributed (copies made mostly of offset slices): a CTA holds its rows and
 //     gathers the others' through distributed shared memory; a stencil's
 //     gathers are contiguous 32-row segments, few of them remote;
-//   replicated (copies with column slices): every CTA holds the whole
+//   replicated (made mostly of column slices): every CTA holds the whole
 //     iterate, gathers from its own memory, and stores each new row into
 //     every CTA's other copy (a contiguous 32-row store per CTA).
 // What bounds a pass is the traffic between the SMs (about 14 bytes per
@@ -1221,6 +1221,7 @@ namespace cg = cooperative_groups;
 constexpr int kClusterWarps = 16;
 constexpr int kClusterThreads = kClusterWarps * 32;
 constexpr int kClusterMax = 8;  // the portable cluster size
+constexpr int32_t kClusterMaxSlices = kClusterMax * 64;  // of a level that may fit one
 constexpr size_t kClusterSmem = 220 * 1024;
 // A pass costs about one dependent shared-memory gather chain per slot of
 // the busiest warp; beyond this many slots a separate launch per sweep over
@@ -1305,11 +1306,12 @@ __device__ __forceinline__ void cluster_store(uint32_t addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
 
-// Form of a level's cluster passes: the iterate distributed or replicated, or
-// (uniform copies) distributed with the uniform slices' row sums.
+// Form of a level's cluster passes: the iterate distributed, or replicated
+// (copies made mostly of column slices), or (uniform copies) distributed with
+// the uniform slices' row sums.
 enum { kClusterDistributed = 0, kClusterReplicated, kClusterUniform };
-inline int cluster_form(bool uniform, bool has_columns) {
-  return uniform ? kClusterUniform : (has_columns ? kClusterReplicated : kClusterDistributed);
+inline int cluster_form(bool uniform, bool direct) {
+  return uniform ? kClusterUniform : (direct ? kClusterReplicated : kClusterDistributed);
 }
 
 template <typename VT, typename XT, int KB, int Form>
@@ -1613,13 +1615,19 @@ bcmg_status cluster_launch_as(const SlicedView &S, const ClusterArgs<XT> &a, cud
 template <typename VT, typename XT, int KB>
 bcmg_status cluster_launch_kb(const SlicedView &S, const ClusterArgs<XT> &a, cudaStream_t st,
                               bool warm_only) {
-  switch (cluster_form(S.uniform != 0, S.cols_staged != 0)) {
-    case kClusterDistributed:
-      return cluster_launch_as<VT, XT, KB, kClusterDistributed>(S, a, st, warm_only);
+  // (kernels only for the batches that copy_batch gives each form)
+  switch (cluster_form(S.uniform != 0, S.direct != 0)) {
     case kClusterReplicated:
-      return cluster_launch_as<VT, XT, KB, kClusterReplicated>(S, a, st, warm_only);
-    default: return cluster_launch_as<VT, XT, KB, kClusterUniform>(S, a, st, warm_only);
+      if constexpr (KB == 8)
+        return cluster_launch_as<VT, XT, KB, kClusterReplicated>(S, a, st, warm_only);
+      break;
+    case kClusterUniform:
+      if constexpr (KB == 8 || KB == uniform_batch<XT>(KB))
+        return cluster_launch_as<VT, XT, KB, kClusterUniform>(S, a, st, warm_only);
+      break;
+    default: return cluster_launch_as<VT, XT, KB, kClusterDistributed>(S, a, st, warm_only);
   }
+  return set_error(BCMG_ERR_INTERNAL, "no cluster kernel of batch %d for this copy", KB);
 }
 
 template <typename VT, typename XT>
@@ -1737,12 +1745,12 @@ bcmg_status warm_kernels(const SlicedView &S) {
 bcmg_status plan_cluster(SlicedMat *out, cudaStream_t s) {
   const int32_t ns = out->nslices;
   out->cl_size = out->cl_spc = out->cl_slots = 0;
-  if (ns <= kClusterMax * 64) {
+  if (ns <= kClusterMaxSlices) {
     std::vector<int32_t> h_sptr(static_cast<size_t>(ns) + 1);
     BCMG_CUDA(cudaMemcpyAsync(h_sptr.data(), out->sptr, sizeof(int32_t) * (ns + 1),
                               cudaMemcpyDeviceToHost, s));
     BCMG_CUDA(cudaStreamSynchronize(s));
-    const bool repl = cluster_form(out->uniform, out->has_columns) == kClusterReplicated;
+    const bool repl = cluster_form(out->uniform, out->direct) == kClusterReplicated;
     int32_t spc = ceil_div(ns, kClusterMax);
     if (!repl) {  // a power of two: the owner of a row is a shift away
       spc = 1;
@@ -1925,10 +1933,11 @@ bcmg_status sliced_build(const CsrView &A, int vtype, SlicedMat *out, cudaStream
   // k_sl_cols where most slots are column slots, except for 16-bit values in
   // narrow slices, which the staged pipeline (32 consumer warps per SM at that
   // size) streams a little faster: 1.2 M rows, 8.4 slots, BF16: 18.4 against
-  // 19.6 us per sweep; from 9.7 slots on the direct form is the faster one.
+  // 19.6 us per sweep; from 9.7 slots on the direct form is the faster one,
+  // and always on levels small enough for a cluster.
   out->direct = !out->uniform && out->has_columns &&
                 2 * static_cast<int64_t>(h_stats[kStatColSlots]) >= slots &&
-                !(value_bytes(vtype) == 2 && out->batch <= 9);
+                !(value_bytes(vtype) == 2 && out->batch <= 9 && ns > kClusterMaxSlices);
   if (out->uniform) {
     launch(k_drop_uniform, ceil_div(ns, 256), 256, 0, s, ns, ukind.get(), width.get());
     BCMG_TRY(exclusive_scan(width.get(), out->sptr, ns, out->sptr + ns, tmp.get(), s));
