@@ -635,6 +635,7 @@ bcmg_status bcmg_level_relax_batch(bcmg_handle *h, int hrc, int level, int32_t w
   const DevLevel &lv = h->H[hrc].lv[level];
   const BtCfg cfg = S.cfg[hrc][level];
   cudaStream_t s = h->stream;
+  pdl_fence(s);  // the caller may have filled f and u by copies on this stream
   if (h->mixed) {
     const float *d = h->prm.relax_type == 0 ? lv.D32 : lv.M32;
     BCMG_TRY(bt_relax<float>(BtLv<float>::mat(lv), width, cfg, d,

@@ -75,6 +75,8 @@ __device__ __forceinline__ void pdl_trigger() {
 // kernels are kernels themselves (copy_t), and an upload that a launch_pdl
 // kernel follows is closed by pdl_fence: an empty kernel launched normally,
 // which starts only after everything before it on the stream has finished.
+// A public call cannot know what its caller put on the stream: one that
+// would begin with a launch_pdl kernel begins with pdl_fence.
 namespace {
 __global__ void k_pdl_fence() {}
 }  // namespace

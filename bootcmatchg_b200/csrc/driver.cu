@@ -2041,6 +2041,7 @@ bcmg_status bcmg_set_stream(bcmg_handle *h, void *stream) {
 bcmg_status bcmg_precond_apply(bcmg_handle *h, const double *d_r, double *d_z) {
   if (!h || !d_r || !d_z) return set_error(BCMG_ERR_PARAM, "null argument");
   BCMG_CUDA(cudaSetDevice(h->device));
+  pdl_fence(h->stream);  // the caller may have filled r and z by copies on this stream
   BCMG_TRY(precond_apply(h, d_r, d_z, false, h->mixed));
   BCMG_CUDA(cudaStreamSynchronize(h->stream));
   return BCMG_OK;
@@ -2120,6 +2121,7 @@ bcmg_status bcmg_level_relax(bcmg_handle *h, int hrc, int level, const void *d_f
   const DevLevel &lv = H.lv[level];
   const bool coarsest = level == static_cast<int>(H.lv.size()) - 1;
   const int type = coarsest ? h->prm.coarse_solver : h->prm.relax_type;
+  pdl_fence(h->stream);  // the caller may have filled f and u by copies on this stream
   if (h->mixed) {
     const float *dd = type == 0 ? Lv<float>::D(lv) : Lv<float>::M(lv);
     BCMG_TRY(relax_t<float>(Lv<float>::mat(lv), dd, static_cast<const float *>(d_f),
