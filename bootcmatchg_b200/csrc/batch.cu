@@ -456,6 +456,7 @@ bcmg_status bt_fcg(bcmg_handle *h, BatchState &S, int m, bcmg_solve_info *infos,
   }
   if (graphs && S.exec) {
     BCMG_CUDA(cudaGraphLaunch(S.exec, s));
+    pdl_fence(s);  // the residual below is a programmatic launch
   } else {
     int any = 1;
     while (any) {

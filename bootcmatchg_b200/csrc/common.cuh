@@ -72,9 +72,10 @@ __device__ __forceinline__ void pdl_trigger() {
 // stream copy or memset just before it is not ordered by its pdl_wait().  A
 // test that ran five sweeps after a device-to-device copy of the iterate
 // read rows the copy had not yet written.  So copies between solve-phase
-// kernels are kernels themselves (copy_t), and an upload that a launch_pdl
-// kernel follows is closed by pdl_fence: an empty kernel launched normally,
-// which starts only after everything before it on the stream has finished.
+// kernels are kernels themselves (copy_t), and whatever else a launch_pdl
+// kernel follows, an upload or a graph launch, is closed by pdl_fence: an
+// empty kernel launched normally, which starts only after everything before
+// it on the stream has finished.
 // A public call cannot know what its caller put on the stream: one that
 // would begin with a launch_pdl kernel begins with pdl_fence.
 namespace {

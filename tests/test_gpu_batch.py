@@ -160,6 +160,27 @@ def test_batch_initial_guess_and_itnlim():
     assert not any(i.converged for i in infos)
 
 
+@pytest.mark.parametrize("graphs", [1, 0])
+@pytest.mark.parametrize("prec", [bc.PREC_FP64, bc.PREC_MIXED])
+def test_true_residual_is_that_of_the_returned_solution(prec, graphs):
+    """The reported true residual is taken after the whole loop: it equals the
+    norm recomputed from the returned columns.  Bound: row sums of m products
+    in any order and the subtraction are within (m + 1) eps of the sum of the
+    magnitudes, on both sides, and the two norms within n eps."""
+    A = wl.poisson(7, 48, 48, 48)
+    B = rhs_block(A.n, list(range(200, 232)))
+    ext = bc.Extensions(precision=prec, use_graphs=graphs, autotune=0,
+                        replace_every=10 if prec == bc.PREC_MIXED else 0)
+    with bc.Handle(A, c1_params(), ext) as h:
+        X, infos = h.solve_batch(B)
+    S, eps = A.to_scipy(), 2.0 ** -53
+    for j in range(B.shape[1]):
+        r, b0 = np.linalg.norm(B[:, j] - S @ X[:, j]), np.linalg.norm(B[:, j])
+        mag = np.linalg.norm(abs(S) @ abs(X[:, j]) + abs(B[:, j]))
+        bound = 2 * 8 * eps * mag + 2 * A.n * eps * r
+        assert abs(infos[j].true_rel_residual * b0 - r) <= bound, j
+
+
 def test_precond_apply_batch_matches_single():
     import torch
     A = wl.poisson(27, 12, 12, 12)
