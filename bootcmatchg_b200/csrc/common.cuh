@@ -83,6 +83,26 @@ __global__ void k_pdl_fence() {}
 }  // namespace
 inline void pdl_fence(cudaStream_t s) { k_pdl_fence<<<1, 1, 0, s>>>(); }
 
+// A read through a __restrict__ pointer, or a read-only load, is not held
+// back by pdl_wait()'s memory clobber: the compiler may take that memory as
+// unchanged for the whole kernel.  So where a launch_pdl kernel reads in such
+// a way what the kernel ahead may have written, the address is formed from a
+// value that passed after_wait(): one the compiler first knows where
+// after_wait stands, below pdl_wait().  Index and lane values do as well as
+// pointers, and keep the pointer's address space and no-alias facts.
+template <typename T>
+__device__ __forceinline__ T after_wait(T v) {
+  if constexpr (sizeof(T) == 8)
+    asm volatile("" : "+l"(v));
+  else
+    asm volatile("" : "+r"(v));
+  return v;
+}
+// The thread's index in the grid, through after_wait().
+__device__ __forceinline__ int64_t thread_after_wait() {
+  return after_wait(static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x);
+}
+
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                        cudaStream_t s, Args &&...args) {

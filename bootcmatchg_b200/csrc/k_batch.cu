@@ -123,7 +123,6 @@ __global__ void __launch_bounds__(256)
   const int L = 1 << lgL;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t gi = t >> lgL;
-  const int g = threadIdx.x & (L - 1);
   const bool valid = gi < n;
   const int32_t i = valid ? static_cast<int32_t>(gi) : 0;
   int32_t j0 = 0;
@@ -135,6 +134,7 @@ __global__ void __launch_bounds__(256)
   // (The matrix is not written by the kernel ahead: its row bounds need not
   // wait for that kernel.)
   pdl_wait();
+  const int g = after_wait(static_cast<int>(threadIdx.x & (L - 1)));
   // The row's own f, u and d do not depend on the row sum: load them first.
   const int64_t o = static_cast<int64_t>(i) * W + static_cast<int64_t>(g) * V;
   Cols<XT, V> fv;
@@ -175,7 +175,7 @@ template <typename XT>
 __global__ void k_bt_relax_zero(int64_t total, int lgW, const XT *__restrict__ d,
                                 const XT *__restrict__ f, XT *__restrict__ out) {
   pdl_wait();
-  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
+  for (int64_t e = thread_after_wait(); e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x)
     out[e] = f[e] / d[e >> lgW];
 }
@@ -185,7 +185,7 @@ __global__ void k_bt_restrict(int32_t nc, int W, int lgL, const int32_t *__restr
                               const int32_t *__restrict__ ridx, const XT *__restrict__ p,
                               const XT *__restrict__ x, XT *__restrict__ y) {
   pdl_wait();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = thread_after_wait();
   const int64_t I = t >> lgL;
   if (I >= nc) return;
   const int64_t cofs = static_cast<int64_t>(threadIdx.x & ((1 << lgL) - 1)) * V;
@@ -210,7 +210,7 @@ __global__ void k_bt_prolong(int32_t n, int W, int lgL, const int32_t *__restric
                              const XT *__restrict__ p, const XT *__restrict__ xc,
                              XT *__restrict__ xf) {
   pdl_wait();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = thread_after_wait();
   const int64_t i = t >> lgL;
   if (i >= n) return;
   const int64_t cofs = static_cast<int64_t>(threadIdx.x & ((1 << lgL) - 1)) * V;
@@ -227,7 +227,6 @@ __global__ void k_bt_prolong(int32_t n, int W, int lgL, const int32_t *__restric
 // reads and the interleaved writes are contiguous.
 __global__ void k_bt_pack(int32_t n, int m, const double *__restrict__ src, int64_t ld,
                           double *__restrict__ dst, int W, int lgW) {
-  pdl_wait();
   __shared__ double tile[32][kBatchMax + 1];
   const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 32;
   const int r = threadIdx.x & 31;
@@ -247,7 +246,7 @@ __global__ void k_bt_unpack(int32_t n, int m, const double *__restrict__ src, in
                             double *__restrict__ dst, int64_t ld) {
   pdl_wait();
   __shared__ double tile[32][kBatchMax + 1];
-  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 32;
+  const int64_t i0 = after_wait(static_cast<int64_t>(blockIdx.x) * 32);
   for (int e = threadIdx.x; e < 32 * W; e += blockDim.x) {
     const int rr = e >> lgW, c = e & (W - 1);
     const int64_t i = i0 + rr;
@@ -316,7 +315,7 @@ __global__ void __launch_bounds__(kRedT)
               const double *__restrict__ c, const double *__restrict__ d, double *partials) {
   pdl_wait();
   double acc[2][1] = {{0.0}, {0.0}};
-  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
+  for (int64_t e = thread_after_wait(); e < total;
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     acc[0][0] = fma(a[e], b[e], acc[0][0]);
     if (c) acc[1][0] = fma(c[e], d[e], acc[1][0]);
@@ -374,7 +373,7 @@ __global__ void __launch_bounds__(kRedT)
   const int L = 1 << lgL;
   const int g = threadIdx.x & (L - 1);
   const int64_t groups = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> lgL;
-  const int64_t g0 = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> lgL;
+  const int64_t g0 = thread_after_wait() >> lgL;
   const int64_t rounds = (n + groups - 1) / groups;
   double acc[3][V];
 #pragma unroll
@@ -471,7 +470,7 @@ __global__ void __launch_bounds__(kRedT)
                     double *partials) {
   pdl_wait();
   double acc[1][1] = {{0.0}};
-  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t0 = thread_after_wait();
   const double *S = scal + (t0 & (W - 1)) * kBtStride;
   if (S[kBtAct] != 0.0) {
     const double theta = S[kTheta];
@@ -503,7 +502,7 @@ __global__ void k_bt_norm_final(const double *partials, double *scal, int W, int
   if (threadIdx.x == 0 && scal[c * kBtStride + key] != 0.0) scal[c * kBtStride + kNorm] = sqrt(s);
 }
 
-// Residual replacement decision per column (as k_fcg_update's); flags[1] says
+// Residual replacement decision per column (k_replace_flag); flags[1] says
 // whether any column replaces.
 __global__ void k_bt_replace_flag(double *scal, int W, int every, int *flags) {
   pdl_wait();
@@ -532,9 +531,9 @@ __global__ void __launch_bounds__(kRedT)
   pdl_wait();
   if (flags[1] == 0) return;  // uniform over the grid
   const int L = 1 << lgL;
-  const int g = threadIdx.x & (L - 1);
+  const int g = after_wait(static_cast<int>(threadIdx.x & (L - 1)));
   const int64_t groups = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> lgL;
-  const int64_t g0 = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> lgL;
+  const int64_t g0 = thread_after_wait() >> lgL;
   const int64_t rounds = (n + groups - 1) / groups;
   bool rep[V];
 #pragma unroll
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(kRedT)
   bt_block_partials<1, V>(acc, W, L, partials);
 }
 
-// End of an iteration per column (fcg_end_iteration): count it, stop the column
+// End of an iteration per column (k_fcg_continue): count it, stop the column
 // when it converged, hit itnlim or broke down; the WHILE condition is "some
 // column still iterating".
 __global__ void k_bt_continue(double *scal, int W, int *flags, cudaGraphConditionalHandle cond,

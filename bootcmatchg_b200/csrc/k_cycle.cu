@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kThreads)
               const XT *__restrict__ f, const XT *__restrict__ u, XT *__restrict__ u_out) {
   pdl_wait();
   pdl_trigger();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = thread_after_wait();
   int32_t i = static_cast<int32_t>(t / G);
   const int lane = threadIdx.x % G;
   if (i >= n) i = -1;
@@ -63,7 +63,7 @@ __global__ void k_relax_zero_t(int32_t n, const XT *__restrict__ d, const XT *__
                                XT *__restrict__ u_out) {
   pdl_wait();
   pdl_trigger();
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t i = static_cast<int32_t>(thread_after_wait());
   if (i < n) u_out[i] = f[i] / d[i];
 }
 
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kThreads)
                  const XT *__restrict__ u, XT *__restrict__ res) {
   pdl_wait();
   pdl_trigger();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = thread_after_wait();
   int32_t i = static_cast<int32_t>(t / G);
   const int lane = threadIdx.x % G;
   if (i >= n) i = -1;
@@ -88,7 +88,7 @@ __global__ void k_restrict_t(int32_t nc, const int32_t *__restrict__ rptr,
                              const XT *__restrict__ x, XT *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const int32_t I = blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t I = static_cast<int32_t>(thread_after_wait());
   if (I >= nc) return;
   XT s = XT(0);
   for (int32_t k = rptr[I]; k < rptr[I + 1]; ++k) {
@@ -106,7 +106,7 @@ __global__ void k_restrict_first_t(int32_t nc, const int32_t *__restrict__ rptr,
                                    const XT *__restrict__ dc, XT *__restrict__ u1) {
   pdl_wait();
   pdl_trigger();
-  const int32_t I = blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t I = static_cast<int32_t>(thread_after_wait());
   if (I >= nc) return;
   XT s = XT(0);
   for (int32_t k = rptr[I]; k < rptr[I + 1]; ++k) {
@@ -123,7 +123,7 @@ __global__ void k_convert_first(int64_t n, const double *__restrict__ in,
                                 float *__restrict__ u1) {
   pdl_wait();
   pdl_trigger();
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+  for (int64_t i = thread_after_wait(); i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const float v = static_cast<float>(in[i]);
     out[i] = v;
@@ -137,7 +137,7 @@ __global__ void k_prolong_t(int32_t n, const int32_t *__restrict__ agg,
                             XT *__restrict__ xf) {
   pdl_wait();
   pdl_trigger();
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t i = static_cast<int32_t>(thread_after_wait());
   if (i < n) xf[i] = fma(p[i], xc[agg[i]], xf[i]);
 }
 
@@ -154,7 +154,7 @@ template <typename XT>
 __global__ void k_axpy_t(int64_t n, XT a, const XT *__restrict__ x, XT *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+  for (int64_t i = thread_after_wait(); i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     y[i] = fma(a, x[i], y[i]);
 }
@@ -164,7 +164,7 @@ template <typename XT>
 __global__ void k_copy_t(int64_t n, const XT *__restrict__ src, XT *__restrict__ dst) {
   pdl_wait();
   pdl_trigger();
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+  for (int64_t i = thread_after_wait(); i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     dst[i] = src[i];
 }
@@ -182,7 +182,7 @@ template <typename From, typename To>
 __global__ void k_convert(int64_t n, const From *__restrict__ in, To *__restrict__ out) {
   pdl_wait();
   pdl_trigger();
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+  for (int64_t i = thread_after_wait(); i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     out[i] = static_cast<To>(in[i]);
 }
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kThreads)
              const VT *__restrict__ val, const XT *__restrict__ x, XT *__restrict__ y) {
   pdl_wait();
   pdl_trigger();
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = thread_after_wait();
   int32_t i = static_cast<int32_t>(t / G);
   const int lane = threadIdx.x % G;
   if (i >= n) i = -1;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kRedThreads)
   pdl_wait();
   pdl_trigger();
   double v[1] = {0.0};
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+  for (int64_t i = thread_after_wait(); i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     v[0] = fma(static_cast<double>(a[i]), static_cast<double>(b[i]), v[0]);
   block_partials<1>(v, partials);

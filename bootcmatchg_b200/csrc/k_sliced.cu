@@ -496,14 +496,6 @@ __device__ __forceinline__ double gather(const double *x, int32_t i) {
   return v;
 }
 
-// p, as a value the compiler first knows here: read-only loads through it
-// cannot move above a pdl_wait() that precedes this call.
-template <typename T>
-__device__ __forceinline__ const T *after_wait(const T *p) {
-  asm volatile("" : "+l"(p));
-  return p;
-}
-
 // Gathers of a row sum from the iterate in global memory: x[i], or x[r + o]
 // relative to the row set by row() (one 64-bit multiply-add per gather).
 template <typename XT>

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kThreads)
   pdl_wait();
   pdl_trigger();
   double v[1] = {0.0};
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+  for (int64_t i = thread_after_wait(); i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     v[0] = fma(a[i], b[i], v[0]);
   block_partials<1>(v, partials);
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kThreads)
   double acc[3] = {0.0, 0.0, 0.0};
   const int lane = threadIdx.x % G;
   const int64_t groups = static_cast<int64_t>(gridDim.x) * blockDim.x / G;
-  const int64_t g0 = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / G;
+  const int64_t g0 = thread_after_wait() / G;
   const int64_t rounds = (n + groups - 1) / groups;
   for (int64_t rd = 0; rd < rounds; ++rd) {
     const int64_t gi = g0 + rd * groups;
@@ -148,14 +148,13 @@ __global__ void __launch_bounds__(kThreads)
     k_fcg_update(int64_t n, int first, const double *__restrict__ z,
                  double *__restrict__ zp, const double *__restrict__ az,
                  double *__restrict__ azp, double *__restrict__ x,
-                 double *__restrict__ r, const double *__restrict__ scal,
-                 double *partials) {
+                 double *__restrict__ r, const double *scal, double *partials) {
   pdl_wait();
   pdl_trigger();
   double acc[1] = {0.0};
   const double theta = scal[kTheta];
   const double theta2 = first ? theta : scal[kTheta2];
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+  for (int64_t i = thread_after_wait(); i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     double zi = z[i], ai = az[i];
     if (!first) {
