@@ -370,7 +370,12 @@ __device__ __forceinline__ void sort_one_row(int32_t i, const int32_t *__restric
 }
 
 // The queued rows of up to kSortRegMax entries, one warp per row (warps take
-// queue entries q, q + all warps, ...).
+// queue entries q, q + all warps, ...).  Rows of at most 32 entries come from
+// k_sort_prefs_group, many of them where a matrix has two row populations, and
+// keep k_sort_prefs' one entry per lane.  Sort phase with k_sort_prefs, with
+// these rows sorted two entries per lane, and as here: 60 % tridiagonal and
+// 40 % 9-point rows (1.2 M) 1.30, 1.38 and 1.17 ms; 80 % 5-point and 20 %
+// 27-point rows (1.2 M) 1.77, 1.88 and 1.75 ms.
 __global__ void __launch_bounds__(kSortWarps * 32)
     k_sort_prefs_mid(const int32_t *__restrict__ mid_rows, const int32_t *__restrict__ n_mid,
                      const int32_t *__restrict__ row, const int32_t *__restrict__ col,
@@ -386,7 +391,9 @@ __global__ void __launch_bounds__(kSortWarps * 32)
     const int32_t i = mid_rows[q];
     const int32_t b = row[i], T = row[i + 1] - b;
     const double ci = C[i], wi = w[i];
-    if (T <= 64)
+    if (T <= 32)
+      sort_row_regs<1>(i, b, T, ci, wi, col, val, w, C, den, W_out, sW, scol, inv, ucnt, lane);
+    else if (T <= 64)
       sort_row_regs<2>(i, b, T, ci, wi, col, val, w, C, den, W_out, sW, scol, inv, ucnt, lane);
     else
       sort_row_regs<4>(i, b, T, ci, wi, col, val, w, C, den, W_out, sW, scol, inv, ucnt, lane);
@@ -430,9 +437,10 @@ __global__ void __launch_bounds__(kSortWarps * 32)
 // most of its lanes idle and its sorting network sized for 32 entries (15
 // exchange steps; 10 for 16, 6 for 8).  Rows of more than G entries go to the
 // queues of the longer sorts.  The order is total, so every path gives the
-// same permutation.  2-D finite volume 2048^2 (5 entries per row, then 6 to 7),
-// three hierarchies: the sorts took 13.2 ms of the setup with k_sort_prefs;
-// the complete solve is 9.3 ms shorter with these (400.9 -> 391.6 ms).
+// same permutation.  Sort phase of one hierarchy's setup, k_sort_prefs and
+// here: 2-D finite volume 1000^2 (5 entries per row, then 6 to 7) 1.65 and
+// 0.95 ms, 5-point 1000^2 1.11 and 0.59 ms (the setups: 6.53 and 5.82 ms,
+// 8.36 and 7.70 ms).
 template <int G>
 __global__ void __launch_bounds__(kSortWarps * 32)
     k_sort_prefs_group(int32_t n, const int32_t *__restrict__ row,
@@ -2026,7 +2034,8 @@ bcmg_status pair_aggregate(const CsrView &A, const double *w, int32_t *agg, doub
   BCMG_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), s));
   BCMG_CUDA(cudaMemsetAsync(nonsym.get(), 0, sizeof(int), s));
   // Lanes per row by the mean row length, with room for rows half as long
-  // again; rows that do not fit are queued.
+  // again; rows that do not fit are queued (k_sort_prefs_mid has the times of
+  // matrices where many do).
   const int64_t mean10 = 10 * static_cast<int64_t>(A.nnz) / n;
   auto sort_rows = [&](auto kernel, int rows_per_warp) {
     launch(kernel, ceil_div(n, kSortWarps * rows_per_warp), kSortWarps * 32, 0, s, n, A.row,
@@ -2039,8 +2048,8 @@ bcmg_status pair_aggregate(const CsrView &A, const double *w, int32_t *agg, doub
     sort_rows(k_sort_prefs_group<16>, 4);
   else
     sort_rows(k_sort_prefs, kSortRowsPerWarp);
-  // Rows of 33..kSortRegMax entries: a grid of a few warps per SM walks the
-  // queue (its length stays on the device).
+  // Queued rows of up to kSortRegMax entries: a grid of a few warps per SM
+  // walks the queue (its length stays on the device).
   launch(k_sort_prefs_mid, std::min(ceil_div(n, kSortWarps), 4 * kNumSM), kSortWarps * 32, 0,
          s, mid_rows.get(), n_mid, A.row, A.col, A.val, w, C.get(), minb.get(), W_out,
          sW.get(), scol.get(), inv.get(), ucnt.get());
