@@ -35,7 +35,8 @@ struct BatchState {
   int W = 0;
   CycleBufs<double> c64;
   CycleBufs<float> c32;
-  // FCG blocks (n x W, FP64, interleaved).
+  // FCG blocks (n x W, FP64, interleaved).  v, the cycle's result, only on
+  // FP64 handles: the mixed-precision cycle leaves it in c32.out0.
   double *r = nullptr, *v = nullptr, *w = nullptr, *d = nullptr, *q = nullptr, *b = nullptr,
          *x = nullptr, *tmp = nullptr;
   double *partials = nullptr, *scal = nullptr, *colnorm = nullptr;
@@ -257,8 +258,9 @@ bcmg_status create_state(bcmg_handle *h, int W) {
   S->W = W;
   h->batch = S;
   const int64_t cnt = static_cast<int64_t>(h->A0.n) * W;
-  for (double **p : {&S->r, &S->v, &S->w, &S->d, &S->q, &S->b, &S->x, &S->tmp})
+  for (double **p : {&S->r, &S->w, &S->d, &S->q, &S->b, &S->x, &S->tmp})
     BCMG_TRY(dev_alloc(p, cnt, s));
+  if (!h->mixed) BCMG_TRY(dev_alloc(&S->v, cnt, s));
   BCMG_TRY(dev_alloc(&S->partials, static_cast<int64_t>(kRedBlocks) * 4 * W, s));
   BCMG_TRY(dev_alloc(&S->scal, static_cast<int64_t>(W) * kBtStride, s));
   BCMG_TRY(dev_alloc(&S->colnorm, W, s));
@@ -515,7 +517,8 @@ size_t batch_bytes(const bcmg_handle *h) {
   if (!h || !h->batch) return 0;
   const BatchState &S = *h->batch;
   const size_t n = static_cast<size_t>(h->A0.n), W = static_cast<size_t>(S.W);
-  return 8 * 8 * n * W + 8 * (4 * static_cast<size_t>(kRedBlocks) * W + W * kBtStride + W) +
+  return 8 * (S.v ? 8 : 7) * n * W +
+         8 * (4 * static_cast<size_t>(kRedBlocks) * W + W * kBtStride + W) +
          cycle_bytes(S.c64, n, W) + cycle_bytes(S.c32, n, W);
 }
 
@@ -612,8 +615,8 @@ bcmg_status bcmg_precond_apply_batch(bcmg_handle *h, int32_t nrhs, const double 
   for (int32_t c0 = 0; c0 < nrhs; c0 += W) {
     const int m = std::min<int32_t>(W, nrhs - c0);
     BCMG_TRY(bt_pack(n, m, d_R + static_cast<int64_t>(c0) * ldr, ldr, S.r, W, s));
-    BCMG_TRY(bt_precond(h, S, S.r, S.v, true));
-    BCMG_TRY(bt_unpack(n, m, S.v, W, d_Z + static_cast<int64_t>(c0) * ldz, ldz, s));
+    BCMG_TRY(bt_precond(h, S, S.r, S.tmp, true));
+    BCMG_TRY(bt_unpack(n, m, S.tmp, W, d_Z + static_cast<int64_t>(c0) * ldz, ldz, s));
   }
   BCMG_CUDA(cudaStreamSynchronize(s));
   return BCMG_OK;
