@@ -2261,6 +2261,7 @@ bcmg_status bcmg_k_relax(int32_t n, int32_t nnz, const int32_t *d_row, const int
   A.val = d_val;
   DevBuf<double> tmp;
   BCMG_TRY(tmp.alloc(n, s));
+  pdl_fence(s);  // the caller may have filled the vectors by copies on this stream
   BCMG_TRY(relax_t<double>(mat_f64(A), d_d, d_f, d_u, tmp.get(), k, false, s));
   BCMG_CUDA(cudaStreamSynchronize(s));
   return BCMG_OK;

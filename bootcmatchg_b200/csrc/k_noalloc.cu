@@ -85,6 +85,7 @@ extern "C" bcmg_status bcmg_k_relax_noalloc(int32_t n, int32_t nnz, const int32_
   A.row = d_row;
   A.col = d_col;
   A.val = d_val;
+  pdl_fence(s);  // the caller may have filled the vectors by copies on this stream
   BCMG_TRY(relax_t<double>(mat_f64(A), d_d, d_f, d_u, scratch, k, false, s));
   BCMG_CUDA(cudaStreamSynchronize(s));
   return BCMG_OK;

@@ -94,6 +94,20 @@ def test_precond_apply(bound):
         block(n * W, torch.float64, 7), block(n * W, torch.float64, 8))
 
 
+@pytest.mark.parametrize("call", ["bcmg_k_relax", "bcmg_k_relax_noalloc"])
+@pytest.mark.parametrize("k", [1, 2])
+def test_single_step_relax(call, k):
+    A = wl.poisson(7, 96, 96, 96)
+    stream = torch.cuda.Stream()
+    m = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (A.row, A.col, A.val)]
+    d = torch.full((A.n,), 13.0, dtype=torch.float64, device="cuda")
+    same_after_copies(
+        stream,
+        lambda f, u: check(getattr(lib, call)(A.n, A.nnz, *map(ptr, m), ptr(d), ptr(f), ptr(u), k,
+                                              C.c_void_p(stream.cuda_stream)), call),
+        block(A.n, torch.float64, 13), block(A.n, torch.float64, 14))
+
+
 def test_solves(bound):
     h, stream, _ = bound
     n = h.n
