@@ -126,6 +126,8 @@ SIGNATURES = {
     "bcmg_level_relax": (C.c_int, [vp, C.c_int, C.c_int, vp, vp, C.c_int]),
     "bcmg_level_format": (C.c_int, [vp, C.c_int, C.c_int, C.POINTER(C.c_int64),
                                     C.POINTER(C.c_int64), i32p, i32p]),
+    "bcmg_level_pass": (C.c_int, [vp, C.c_int, C.c_int, C.POINTER(C.c_int), i32p, i32p,
+                                  C.POINTER(C.c_int)]),
     "bcmg_k_pair_aggregate": (C.c_int, [i32, i32, vp, vp, vp, vp, vp, vp, i32p, vp, vp,
                                         vp, vp]),
     "bcmg_k_spgemm": (C.c_int, [i32, i32, i32, vp, vp, vp, i32, i32, vp, vp, vp, vp, i32p,

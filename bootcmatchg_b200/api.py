@@ -143,6 +143,9 @@ class Params:
         check(lib.bcmg_params_check(C.byref(p)), "Params.check")
 
 
+PASS_NAMES = ("csr", "staged", "columns", "uniform")  # BCMG_PASS_*
+
+
 @dataclass
 class Extensions:
     precision: int = PREC_FP64
@@ -347,6 +350,15 @@ class Handle:
                                       C.byref(ac)), "hierarchy_info")
         return {"num_levels": nl.value, "op_cmplx": oc.value, "op_wcmplx": ow.value,
                 "avg_cratio": ac.value}
+
+    def level_pass(self, hrc: int, level: int) -> dict:
+        """The kernel that runs the level's row passes (PASS_NAMES), its
+        uniform slices and those with masks, and the CTAs of its cluster."""
+        f, u, m, c = C.c_int(), C.c_int32(), C.c_int32(), C.c_int()
+        check(lib.bcmg_level_pass(self._h, hrc, level, C.byref(f), C.byref(u), C.byref(m),
+                                  C.byref(c)), "level_pass")
+        return {"pass": PASS_NAMES[f.value], "uniform_slices": u.value,
+                "masked_slices": m.value, "cluster_ctas": c.value}
 
     def level(self, hrc: int, level: int) -> LevelData:
         n, nnz, nc = C.c_int32(), C.c_int32(), C.c_int32()

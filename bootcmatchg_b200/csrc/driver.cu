@@ -2136,6 +2136,18 @@ bcmg_status bcmg_level_relax(bcmg_handle *h, int hrc, int level, const void *d_f
   return sliced_wait_status(h->stream);
 }
 
+// The copy's slice metadata (see SlicedView), on the host.
+static bcmg_status slice_meta(const bcmg_handle *h, const SlicedMat *S, std::vector<int4> *meta) {
+  meta->clear();
+  if (!S || !S->nslices) return BCMG_OK;
+  meta->resize(S->nslices);
+  BCMG_CUDA(cudaSetDevice(h->device));
+  BCMG_CUDA(cudaMemcpyAsync(meta->data(), S->meta, sizeof(int4) * S->nslices,
+                            cudaMemcpyDeviceToHost, h->stream));
+  BCMG_CUDA(cudaStreamSynchronize(h->stream));
+  return BCMG_OK;
+}
+
 bcmg_status bcmg_level_format(const bcmg_handle *h, int hrc, int level, int64_t *slots,
                               int64_t *column_slots, int32_t *slices, int32_t *value_bytes) {
   if (!h || hrc < 0 || hrc >= static_cast<int>(h->H.size()))
@@ -2151,15 +2163,39 @@ bcmg_status bcmg_level_format(const bcmg_handle *h, int hrc, int level, int64_t 
     *value_bytes = !S ? 0 : (S->vtype == kValF64 ? 8 : (S->vtype == kValF32 ? 4 : 2));
   if (column_slots) {
     *column_slots = 0;
-    if (S && S->nslices) {
-      std::vector<int4> meta(S->nslices);
-      BCMG_CUDA(cudaSetDevice(h->device));
-      BCMG_CUDA(cudaMemcpyAsync(meta.data(), S->meta, sizeof(int4) * S->nslices,
-                                cudaMemcpyDeviceToHost, h->stream));
-      BCMG_CUDA(cudaStreamSynchronize(h->stream));
-      for (int32_t i = 0; i < S->nslices; ++i)
-        if (!meta[i].z) *column_slots += meta[i].y;
+    std::vector<int4> meta;
+    BCMG_TRY(slice_meta(h, S, &meta));
+    for (const int4 &m : meta)
+      if (!m.z) *column_slots += m.y;
+  }
+  return BCMG_OK;
+}
+
+bcmg_status bcmg_level_pass(const bcmg_handle *h, int hrc, int level, int *pass,
+                            int32_t *uniform_slices, int32_t *masked_slices,
+                            int *cluster_ctas) {
+  if (!h || hrc < 0 || hrc >= static_cast<int>(h->H.size()))
+    return set_error(BCMG_ERR_PARAM, "bad hierarchy index");
+  const DevHierarchy &H = h->H[hrc];
+  if (level < 0 || level >= static_cast<int>(H.lv.size()))
+    return set_error(BCMG_ERR_PARAM, "bad level index");
+  const DevLevel &lv = H.lv[level];
+  const SlicedMat *S = h->mixed ? slicedlo(lv) : sliced64(lv);
+  if (pass)
+    *pass = !S ? BCMG_PASS_CSR
+               : (S->uniform ? BCMG_PASS_UNIFORM
+                             : (S->direct ? BCMG_PASS_COLUMNS : BCMG_PASS_STAGED));
+  if (cluster_ctas) *cluster_ctas = S ? S->cl_size : 0;
+  if (uniform_slices || masked_slices) {
+    std::vector<int4> meta;
+    BCMG_TRY(slice_meta(h, S, &meta));
+    int32_t uniform = 0, masked = 0;
+    for (const int4 &m : meta) {
+      uniform += m.z >= 4;
+      masked += m.z > 4;
     }
+    if (uniform_slices) *uniform_slices = uniform;
+    if (masked_slices) *masked_slices = masked;
   }
   return BCMG_OK;
 }

@@ -363,6 +363,17 @@ bcmg_status bcmg_level_relax(bcmg_handle *h, int hrc, int level, const void *d_f
 bcmg_status bcmg_level_format(const bcmg_handle *h, int hrc, int level,
                               int64_t *slots, int64_t *column_slots,
                               int32_t *slices, int32_t *value_bytes);
+/* The kernel that runs one level's row passes (no counterpart in the
+ * reference), as the copy's contents chose it: from CSR; the staged pipeline;
+ * the kernel of column-slice copies; the kernel of constant-coefficient
+ * copies.  uniform_slices: slices that store no slots; masked_slices: those
+ * of them whose pass reads one mask word per row; cluster_ctas: CTAs of the
+ * thread-block cluster that runs all sweeps of a small level in one launch
+ * (0: a launch per sweep).  Any output may be NULL. */
+enum { BCMG_PASS_CSR = 0, BCMG_PASS_STAGED = 1, BCMG_PASS_COLUMNS = 2, BCMG_PASS_UNIFORM = 3 };
+bcmg_status bcmg_level_pass(const bcmg_handle *h, int hrc, int level, int *pass,
+                            int32_t *uniform_slices, int32_t *masked_slices,
+                            int *cluster_ctas);
 
 /* ---- single-step entry points on device pointers --------------------------
  * Used by the parity tests; stream may be NULL (legacy default stream).

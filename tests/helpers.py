@@ -40,3 +40,18 @@ def random_sym_graph(n, deg, seed, int_weights=True, diag_shift=1.0):
     a = a.tocsr()
     a.sort_indices()
     return bc.CsrMatrix.from_scipy(a)
+
+
+def varying_stencil(points, nx, ny, nz, seed, ints=False):
+    """The pattern of wl.poisson with coefficients that differ from entry to
+    entry; small integers (exact in BF16) or uniform in [0.5, 2)."""
+    import bootcmatchg_b200 as bc
+    import scipy.sparse as sp
+    import workloads as wl
+    U = sp.triu(wl.poisson(points, nx, ny, nz).to_scipy(), 1).tocsr()
+    rng = np.random.default_rng(seed)
+    U.data = -(rng.integers(1, 4, U.nnz).astype(float) if ints
+               else rng.uniform(0.5, 2.0, U.nnz))
+    S = (U + U.T).tocsr()
+    return bc.CsrMatrix.from_scipy(
+        (S + sp.diags(np.asarray(abs(S).sum(axis=1)).ravel() + 1.0)).tocsr())

@@ -28,7 +28,7 @@ import pytest
 import bootcmatchg_b200 as bc
 import workloads as wl
 from bootcmatchg_b200._lib import lib
-from helpers import c1_params
+from helpers import c1_params, varying_stencil
 
 pytestmark = pytest.mark.gpu
 
@@ -57,14 +57,19 @@ def test_bounded_wait_runs_out_and_device_stays_usable():
 
 
 @pytest.mark.parametrize("prec", [bc.PREC_FP64, bc.PREC_MIXED])
-def test_wait_bound_change_keeps_results(prec):
+@pytest.mark.parametrize("case", ["poisson27_32", "vary27", "vary7"])
+def test_wait_bound_change_keeps_results(case, prec):
     """bcmg_set_max_device_seconds on a live handle (the captured FCG loop is
-    rebuilt with the new bound): same bits as a fresh handle."""
-    A = wl.poisson(27, 32, 32, 32)
+    rebuilt with the new bound): same bits as a fresh handle.  The level-0
+    passes run the pipeline whose waits the bound is for."""
+    A = {"poisson27_32": lambda: wl.poisson(27, 32, 32, 32),
+         "vary27": lambda: varying_stencil(27, 32, 31, 30, 1),
+         "vary7": lambda: varying_stencil(7, 40, 39, 38, 2)}[case]()
     b = wl.vector(1, 1, A.n)
     p = c1_params()
     ext = bc.Extensions(precision=prec, replace_every=10 if prec else 0)
     with bc.Handle(A, p, ext) as h0:
+        assert h0.level_pass(0, 0)["pass"] == "staged"
         x0, i0 = h0.solve(b)
     with bc.Handle(A, p, ext) as h:
         x1, i1 = h.solve(b)

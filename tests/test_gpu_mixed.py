@@ -11,7 +11,7 @@ import pytest
 
 import bootcmatchg_b200 as bc
 import workloads as wl
-from helpers import c1_params
+from helpers import c1_params, random_sym_graph, varying_stencil
 from oracle import oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -115,14 +115,19 @@ def test_sliced_and_csr_solves_agree():
 
 
 @pytest.mark.parametrize("prec", [bc.PREC_FP64, bc.PREC_MIXED])
-def test_exact_value_narrowing_is_bit_identical(prec):
+@pytest.mark.parametrize("case", ["poisson27_32", "vary27_ints", "vary7_ints", "rand_ints"])
+def test_exact_value_narrowing_is_bit_identical(case, prec):
     """Solve-phase copies (the FP64 or FP32 cycle, and the FCG SpMV in both
     modes) store a level's values in BF16 when every value converts exactly
-    (the 27-point stencil's 26 and -1); the kernels widen them, so the
-    solution matches the unnarrowed run bit for bit."""
+    (the 27-point stencil's 26 and -1; small integers); the kernels widen
+    them, so the solution matches the unnarrowed run bit for bit.  No case's
+    level 0 is stored as a constant stencil, which streams no values."""
     import ctypes as C
     from bootcmatchg_b200._lib import check, lib
-    A = wl.poisson(27, 32, 32, 32)
+    A = {"poisson27_32": lambda: wl.poisson(27, 32, 32, 32),
+         "vary27_ints": lambda: varying_stencil(27, 31, 30, 29, 1, ints=True),
+         "vary7_ints": lambda: varying_stencil(7, 41, 40, 39, 2, ints=True),
+         "rand_ints": lambda: random_sym_graph(20001, 12, seed=3)}[case]()
     p = c1_params()
     b = wl.vector(1, 5, A.n)
     out = []
@@ -135,6 +140,7 @@ def test_exact_value_narrowing_is_bit_identical(prec):
             nsl, vb = C.c_int32(), C.c_int32()
             check(lib.bcmg_level_format(h.ptr, 0, 0, C.byref(slots), C.byref(cslots),
                                         C.byref(nsl), C.byref(vb)), "level_format")
+            assert h.level_pass(0, 0)["pass"] == ("columns" if case == "rand_ints" else "staged")
         assert info.converged
         out.append((x, info.iters, vb.value))
     assert out[0][2] == 2
