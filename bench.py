@@ -530,27 +530,31 @@ def run_ours(args):
                                sweeps), "level_relax")
     r1.record(stream)
     torch.cuda.synchronize(dev)
+    rows = h.level_pass(0, 0)
     h.close()
     sweep_s = r0.elapsed_time(r1) / 1e3 / sweeps
+    # the kernel that ran, and what bounds it
+    kernel, bound = {"csr": ("k_relax_t", "hbm"), "staged": ("k_sl_pipe", "hbm"),
+                     "columns": ("k_sl_cols", "l1"),
+                     "uniform": ("k_sl_uniform", "latency")}[rows["pass"]]
     if vbytes.value:
         # sliced copy: values incl. padding (none in constant-coefficient
-        # slices), explicit columns, per-slice metadata, and u (gathered
-        # once), f, d read + u' written
-        sweep_bytes = (vbytes.value * 32 * slots.value + 4 * 32 * cslots.value +
-                       16 * nsl.value + 4 * xbytes * A.n)
-        kname = ("k_sl_uniform<EpiRelax> (level-0 l1-Jacobi sweep, constant stencil)"
-                 if 4 * slots.value < nsl.value else
-                 "k_sl_pipe or k_sl_cols<EpiRelax> (level-0 l1-Jacobi sweep, sliced copy)")
+        # slices, one mask word per row in those that miss entries), explicit
+        # columns, per-slice metadata, and u (gathered once), f, d read + u'
+        # written
+        sweep_bytes = (vbytes.value * 32 * slots.value + 128 * rows["masked_slices"] +
+                       4 * 32 * cslots.value + 16 * nsl.value + 4 * xbytes * A.n)
+        kname = f"{kernel}<EpiRelax> (level-0 l1-Jacobi sweep, {rows['pass']} sliced copy)"
     else:
         sweep_bytes = 12 * A.nnz + 4 * (A.n + 1) + 36 * A.n
         kname = "k_relax_t (level-0 l1-Jacobi sweep, CSR)"
     csr_equiv = 12 * A.nnz + 4 * (A.n + 1) + 36 * A.n
     achieved = sweep_bytes / sweep_s / 1e9
     peak, peak_kind = measured_peaks()
-    # keyed by the copy's value width: a capture of another storage format
-    # (FP32 values, BF16 values) does not describe this launch
-    traffic = committed_traffic("k_sl_pipe",
-                                f"{args.workload}:{args.precision}:{vbytes.value}B")
+    # keyed by the kernel and, where it streams values, their width: a capture
+    # of another kernel or storage format does not describe this launch
+    width = "" if rows["pass"] == "uniform" else f":{vbytes.value}B"
+    traffic = committed_traffic(kernel, f"{args.workload}:{args.precision}{width}")
 
     cpu, err = None, {}
     if world == 1 and rank == 0 and not args.no_cpu_baseline:
@@ -588,7 +592,7 @@ def run_ours(args):
         "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "gpu_launches": int(launches),
-        "roofline": {"kernel": kname, "bound": "hbm",
+        "roofline": {"kernel": kname, "bound": bound,
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind,
                      "traffic": traffic, "algorithmic_bytes": sweep_bytes,
@@ -1057,7 +1061,7 @@ def run_case(args):
                  96): matching, aggregation and Galerkin kernels
 
     Each case sets up its hierarchy first and then runs the kernels of
-    interest; filter on kernel names such as k_sl_pipe or k_bt_rowop."""
+    interest; filter on kernel names such as k_sl_uniform or k_bt_rowop."""
     import torch
 
     import bootcmatchg_b200 as bc

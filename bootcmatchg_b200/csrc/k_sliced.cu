@@ -3,29 +3,41 @@
 // Rows are cut into slices of 32 (one warp, one thread per row).  A slice
 // stores W slots of 32 values in slot-major order, so every slot of a slice
 // is one contiguous 32-element segment and a slice is one contiguous block.
-// Two slot kinds:
+// Three kinds of slices:
 //   offset slice: the slice's rows share a set of W column offsets
 //                 (col - row), e.g. a stencil; column indices are implicit
 //                 (row + offset) and W offsets are stored per slice.  Runs of
 //                 consecutive slices with identical offset lists read one
 //                 copy (the run head's), which stays cache-resident;
-//   column slice: W = longest row; explicit int32 columns per slot (SELL-32).
+//   column slice: W = longest row; explicit int32 columns per slot (SELL-32);
+//   uniform slice: only in a uniform copy, one most of whose slices hold a
+//                 stencil with one coefficient per offset; no slots at all,
+//                 one word per row with the offsets the row has.
 // Missing entries are stored as 0 (with an in-range column), which adds exact
 // zeros to the row sums.  Values, columns and offsets are padded by kSlotPad
 // slots so a batch of loads may run past a slice's last slot without a bounds
 // test (those products are discarded).  Built on the device from the level's
 // CSR after setup; CSR stays the setup / introspection format.
 //
-// Row passes (smoother sweep, residual, SpMV, FCG SpMV + dots) run as one
-// warp-specialised pipeline per CTA: a producer warp streams each chunk of
-// kPipeWarps consecutive slices (values, explicit columns, slice metadata and
-// the row vectors the epilogue reads) into shared memory with bulk async
-// copies (cp.async.bulk, the TMA engine) under full/empty mbarriers, while the
-// kPipeWarps consumer warps compute the previous chunks.  A consumer warp
-// issues all gathers of a batch of slots before its first FMA, so each warp
-// keeps a full row's gathers in flight.  Every wait is bounded; a wait that
-// runs out sets a device error word (sliced_wait_status) and the kernel
-// returns without touching the stage.
+// Row passes (smoother sweep, residual, SpMV, FCG SpMV + dots) run as one of
+// three kernels, by what the copy is made of (pipe_launch):
+//   k_sl_pipe     copies of offset slices: a warp-specialised pipeline per
+//                 CTA.  A producer warp streams each chunk of kPipeWarps
+//                 consecutive slices (values, explicit columns, slice metadata
+//                 and the row vectors the epilogue reads) into shared memory
+//                 with bulk async copies (cp.async.bulk, the TMA engine) under
+//                 full/empty mbarriers, while the kPipeWarps consumer warps
+//                 compute the previous chunks.  A consumer warp issues all
+//                 gathers of a batch of slots before its first FMA.  Every
+//                 wait is bounded; a wait that runs out sets a device error
+//                 word (sliced_wait_status) and the kernel returns without
+//                 touching the stage;
+//   k_sl_cols     copies made mostly of column slices: a warp per slice,
+//                 nothing staged;
+//   k_sl_uniform  uniform copies: a warp per slice, offsets and coefficients
+//                 from the kernel's parameters.
+// A level that fits the shared memory of one thread-block cluster runs all
+// its sweeps in one launch of k_sl_cluster.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -997,12 +1009,14 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_min_blocks<XT, KB>())
 // row vectors (and one mask word per row where some entry is missing), so
 // nothing is staged; a warp per slice gathers through L1, 27 (FP32 vectors)
 // or 9 (FP64) loads in flight per lane with 32 warps per SM.  27-point 128^3:
-// 33.5 MB instead of 146.7 per FP32 sweep; what bounds it now is instruction
-// issue (about 180 per 32 rows: a load, an address or half of one and a
-// multiply-add per slot, bit tests where entries are missing, the division).
+// 38.9 MB instead of 146.7 per FP32 sweep (four vectors 33.6, metadata 1.0,
+// masks of 33,784 of the 65,536 slices 4.3).  No unit is saturated: 177
+// instructions per 32 rows (a load, an address or half of one and a
+// multiply-add per slot, bit tests where entries are missing, the division)
+// take 55 % of the issue slots, the rest waits for gathers (L1 hits 75 %).
 // Per sweep, against the staged pipeline with 16-bit values: level 0 31.3 ->
-// 18.0 us (FP32) and 39.2 -> 26.8 us (FP64), its 524 K-row level 9.3 -> 6.6
-// and 11.6 -> 8.5, 131 K rows 4.35 -> 2.7 and 5.4 -> 3.4.  Fewer loads in
+// 18.0 us (FP32) and 39.2 -> 25.5 us (FP64), its 524 K-row level 9.3 -> 6.6
+// and 11.6 -> 8.4, 131 K rows 4.35 -> 2.7 and 5.4 -> 3.2.  Fewer loads in
 // flight with more warps in FP32 (9 or 14, 40 to 48 warps): 29 us.
 template <typename VT, typename XT, typename Epi, int W>
 __global__ void __launch_bounds__(kPipeWarps * 32, 4)

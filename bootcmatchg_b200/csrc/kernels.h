@@ -61,7 +61,9 @@ enum ValType { kValF64 = 0, kValF32 = 1, kValBF16 = 2, kValF16 = 3 };
 // Sliced solve-phase format (k_sliced.cu): 32-row slices, slot-major values.
 // meta[s] = {first slot, width W, kind, offset base}: kind 1 = shared column
 // offsets soff[base + k] (base = the first slice of a run of slices with the
-// same offsets); kind 0 = explicit columns scol[32 first + 32 k + lane].
+// same offsets), 2 and 3 interior ones (every row + offset in range; 3 with
+// the copy's stencil), 4 to 6 uniform slices (SlicedView); kind 0 = explicit
+// columns scol[32 first + 32 k + lane].
 // Values, columns and offsets are padded past the last slot.
 // Default bound on each wait of a pipelined row pass for its staged copies
 // (bcmg_ext.max_device_seconds overrides it per handle).
@@ -87,8 +89,8 @@ struct SlicedView {
   // CTA and the slot capacity of one CTA's shared memory.
   int32_t cl_size = 0, cl_spc = 0, cl_slots = 0;
   // Stencil slices (meta.z == 3): interior offset slices whose offsets are
-  // exactly sten_off[0 .. sten_w), sten_w being the slot batch of the copy;
-  // the kernels take those offsets from their parameters.
+  // exactly sten_off[0 .. sten_w), those of the first interior slice as wide
+  // as the mean slice; the kernels take them from their parameters.
   int32_t sten_w = 0;
   int32_t sten_off[kStencilMax] = {};
   // Uniform copies (uniform != 0): most slices have one coefficient per
