@@ -58,11 +58,13 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
 
 // Programmatic dependent launch (solve-phase kernels): a kernel launched with
 // launch_pdl may begin while the previous kernel on its stream is still
-// running.  Every such kernel calls pdl_wait() first — it returns once the
-// previous grid has completed and its writes are visible (a no-op for a
-// normal launch) — and pdl_trigger() to let the next one start launching;
-// a grid can only start after every CTA of its predecessor has triggered or
-// exited, so those CTAs are all resident already.
+// running.  Every such kernel calls pdl_wait() before it reads or writes what
+// that kernel may touch — the call returns once the previous grid has
+// completed and its writes are visible (a no-op for a normal launch) — and,
+// except for the batched kernels (k_batch.cu says why), pdl_trigger() after it
+// to let the next one start launching; a grid can only start after every CTA
+// of its predecessor has triggered or exited, so those CTAs are all resident
+// already.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
